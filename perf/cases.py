@@ -474,6 +474,10 @@ def tolerance(case: dict) -> dict:
     """32-bit sums of some hundred terms, about four times the distance seen from ``exact``. The exact mode takes its chords
     from 32-bit slab crossings: few rays through each voxel (pixels coarser than voxels, few views) leave their errors unaveraged."""
     op = case["op"]
+    nearest = op in ("sirt", "fan_fbp") or case.get("mode") in ("nearest", "raycast") or case.get("interpolate") is False
+    if nearest and case.get("nx", case.get("n", 0)) % 2 and case.get("ny", case.get("n", 0)) % 2 and case["nu"] % 2 == 0:
+        # the axis of an odd grid lies on the edge between two detector columns in every view: either is its nearest one
+        return dict(rel=6e-4, max=0.5)
     if op == "project":
         return dict(rel=2e-6, max=4e-3)
     if op == "quadric":
