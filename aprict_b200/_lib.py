@@ -37,6 +37,9 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
         _c_int,
         [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     ),
+    "aprict_b200_backproject_views": (
+        _c_int, [_c_void_p] * 7 + [ctypes.c_uint32, _c_void_p, _c_void_p],
+    ),
     "aprict_b200_vol_fill": (_c_int, [_c_void_p, ctypes.c_int64, ctypes.c_float, _c_void_p]),
     "aprict_b200_vol_scale": (_c_int, [_c_void_p, ctypes.c_int64, ctypes.c_float, _c_void_p]),
     "aprict_b200_vol_invert": (_c_int, [_c_void_p, ctypes.c_int64, _c_int, ctypes.c_float, _c_void_p]),
@@ -102,6 +105,9 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "aprict_b200_sirt_graph_iterations": (_c_int, [_c_void_p]),
     "aprict_b200_sirt_graph_destroy": (None, [_c_void_p]),
     "aprict_b200_batch_plan_bytes": (ctypes.c_size_t, [_c_int, _c_int]),
+    "aprict_b200_batch_plan_views": (
+        _c_int, [_c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, ctypes.c_size_t],
+    ),
     "aprict_b200_batch_plan": (_c_int, [_c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, ctypes.c_size_t]),
     "aprict_b200_batch_run": (_c_int, [_c_void_p, _c_void_p, _c_void_p]),
     "aprict_b200_batch_run_static": (_c_int, [_c_void_p, _c_void_p]),

@@ -37,7 +37,7 @@ def _stream() -> int:
 class BatchPlan:
     """A planned batch operation: the host image and its device copy."""
 
-    def __init__(self, op: int, scans: np.ndarray, configs: np.ndarray, keepalive: list) -> None:
+    def __init__(self, op: int, scans: np.ndarray, configs: np.ndarray, keepalive: list, views: np.ndarray | None = None) -> None:
         lib = _lib.lib()
         n = int(scans.shape[0])
         nbytes = int(lib.aprict_b200_batch_plan_bytes(op, n))
@@ -48,7 +48,10 @@ class BatchPlan:
         off = (-raw.ctypes.data) % 256
         self._host = raw[off : off + nbytes]
         _lib.check(
-            lib.aprict_b200_batch_plan(op, _lib.ptr(scans), n, _lib.ptr(configs), self._host.ctypes.data, nbytes),
+            lib.aprict_b200_batch_plan_views(
+                op, _lib.ptr(scans), n, _lib.ptr(configs), None if views is None else _lib.ptr(views), self._host.ctypes.data,
+                nbytes,
+            ),
             "batch_plan",
         )
         self._dev = _lib.upload(self._host)
@@ -181,7 +184,8 @@ class ScanBatch:
                 msg = "Backprojection weighting preset 7 (the GBC formula) is not implemented."
                 raise NotImplementedError(msg)
         conf = _packed([c.contents for c in cfgs], S.backproject_config)
-        return BatchPlan(BACKPROJECT, recs, conf, keep)
+        views = np.array([p._backproject_promise(c.needs_z) for p, c in zip(self.projs, cfgs, strict=True)], np.uint32)  # noqa: SLF001
+        return BatchPlan(BACKPROJECT, recs, conf, keep, views)
 
     def project(self, configs=None, *, bases=None, block: bool = False) -> None:
         """Plan and run one batched projection."""

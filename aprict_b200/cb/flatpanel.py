@@ -376,6 +376,7 @@ class ProjectionSet:
         self._proj_specs = proj_specs
         self._data = data
         self._specs_dev: torch.Tensor | None = None
+        self._kinds: tuple[bool, bool] | None = None
         self._out_of_mem_counter: torch.Tensor | None = None
 
     def _with_data(self, data: torch.Tensor) -> ProjectionSet:
@@ -387,6 +388,7 @@ class ProjectionSet:
         out._proj_specs = self._proj_specs
         out._data = data
         out._specs_dev = self.specs_device()
+        out._kinds = self._kinds
         out._out_of_mem_counter = None
         return out
 
@@ -434,6 +436,15 @@ class ProjectionSet:
             self._specs_dev = _lib.upload(raw)
         return self._specs_dev
 
+    def _backproject_promise(self, needs_z: bool) -> int:
+        """What the packed views let a backprojection promise (``aprict_b200_backproject_views``)."""
+        if self._kinds is None:
+            sp = self._proj_specs
+            up = (sp["det_u"]["z"] == 0) & (sp["det_v"]["x"] == 0) & (sp["det_v"]["y"] == 0)
+            self._kinds = (bool(up.all()), bool((sp["det_pos"]["z"] == sp["source_pos"]["z"]).all()))
+        upright, level = self._kinds
+        return 1 if upright and (level or not needs_z) else 2
+
     def create_buffer(self, *, dtype: type | np.dtype = np.float32, existing_ok: bool = False) -> None:
         """Allocate a zero-filled data buffer."""
         if self._data is not None:
@@ -453,7 +464,7 @@ class ProjectionSet:
             msg = "Cannot create a zeroed copy without an explicit 'dtype' argument, because the object you are trying to copy does not yet have a determined dtype."
             raise ValueError(msg)
         ps = ProjectionSet(self._proj_geom, data=None)
-        ps._specs_dev = self._specs_dev
+        ps._specs_dev, ps._kinds = self._specs_dev, self._kinds
         ps.create_buffer(dtype=_np_dtype(self._data) if dtype is None else dtype)
         return ps
 
@@ -553,6 +564,12 @@ class ConfigBackproject:
         """The packed aprict_backproject_config."""
         return self._contents.copy()
 
+    @property
+    def needs_z(self) -> bool:
+        """Whether the weights depend on a voxel's distance along the source-detector axis."""
+        c = self._contents
+        return bool(c["Z_on_L_factor_power"] or c["Z_on_val_factor_power"] or c["weighting_preset"])
+
 
 # --------------------------------------------------------------------------- operators
 def _leading_slices(projs: ProjectionSet) -> list[tuple[tuple[int, ...], int]]:
@@ -581,7 +598,7 @@ def _f32_twin(projs: ProjectionSet) -> ProjectionSet:
     if projs.data.dtype == torch.float32:
         return projs
     tw = ProjectionSet(projs.proj_geom, data=torch.zeros(projs.data.shape, dtype=torch.float32, device=projs.data.device))
-    tw._specs_dev = projs._specs_dev  # noqa: SLF001
+    tw._specs_dev, tw._kinds = projs._specs_dev, projs._kinds  # noqa: SLF001
     tw._out_of_mem_counter = projs.out_of_mem_counter  # noqa: SLF001
     return tw
 
@@ -728,11 +745,12 @@ def backproject(
         if block:
             torch.cuda.current_stream().synchronize()
         return volume
+    views = projs._backproject_promise(config.needs_z)  # noqa: SLF001
     for it, first in _leading_slices(projs):
         specs, pd, dptr = _view_args(projs, it, first, data=p32)
         _lib.check(
-            _lib.lib().aprict_b200_backproject(
-                specs, _lib.ptr(pd), dptr, _lib.ptr(vd), v32.data_ptr(), mptr, _lib.ptr(cfg), None, _stream()
+            _lib.lib().aprict_b200_backproject_views(
+                specs, _lib.ptr(pd), dptr, _lib.ptr(vd), v32.data_ptr(), mptr, _lib.ptr(cfg), views, None, _stream()
             ),
             "backproject",
         )

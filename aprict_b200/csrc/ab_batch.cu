@@ -22,12 +22,12 @@
 #include <numeric>
 #include <vector>
 
-#include "ab_bpbrick.cuh"
+#include "ab_bpcol.cuh"
 #include "ab_fptile.cuh"
 
 namespace {
 
-constexpr uint32_t kPlanMagic = 0x41424232u;  // "ABB2"
+constexpr uint32_t kPlanMagic = 0x41424233u;  // "ABB3"
 constexpr int kGroup = 96;                    // scans per launch (kernel-parameter space)
 
 // Plan layout (host image; the caller's device copy is used only for the
@@ -51,6 +51,7 @@ struct Group {
     uint32_t count;    // scans in the group
     uint32_t n_units;
     int32_t grid;                 // persistent CTAs (SMs x resident CTAs, at most n_units)
+    int32_t col_grid;             // the same for the z-column launch
     uint32_t prefix[kGroup + 1];  // cumulative work units of the group's scans
 };
 
@@ -148,20 +149,44 @@ constexpr int batch_xb(int ord, bool exact) { return ord == 2 ? 4 : ab_bp::defau
 // a brick misses the detector: batches mix helical and circular scans, and
 // the helical ones leave most of a volume off each view's detector (48
 // uneven scans: 326.6 -> 265.3 ms per batched backprojection).
-template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, int XB = batch_xb(ORD, EXACT)>
+// COLS: leave the scans that take the z columns to k_batch_columns.
+template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, bool COLS, int XB = batch_xb(ORD, EXACT)>
 __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::bp_min_blocks(XB, EXACT))
     k_batch_backproject(const __grid_constant__ BatchArgs<ab_bp::BPParams> A) {
-    __shared__ ab_bp::BPSmem<EXACT, BILIN, XB, ab_bp::bp_ztable(ORD, EXACT, RAYCAST, BILIN)> sm;
+    __shared__ ab_bp::BPSmem<EXACT, BILIN, XB> sm;
     uint32_t unit;
     int s;
-    while (next_unit(A, unit, s)) ab_bp::bp_brick<ORD, EXACT, RAYCAST, BILIN, XB, true>(A.scans[s], unit, sm);
+    while (next_unit(A, unit, s)) {
+        if (COLS && ab_bp::all_upright(A.scans[s])) continue;
+        ab_bp::bp_brick<ORD, EXACT, RAYCAST, BILIN, XB, true>(A.scans[s], unit, sm);
+    }
+    retire(A.g);
+}
+
+// Batches of the fast modes on volumes of more than one layer run
+// as two launches over the same units: the scans whose views are all upright
+// take the z columns (8 voxels per thread whatever the scan's height; blocks
+// above a volume are skipped), the others the bricks. Each launch passes over
+// the other's units, after reading their views' records where the plan's maker
+// promised nothing; a batch of scans promised general is one launch.
+template <bool RAYCAST, bool BILIN>
+__global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::kColBlocks)
+    k_batch_columns(const __grid_constant__ BatchArgs<ab_bp::BPParams> A) {
+    __shared__ ab_bp::ColSmem<8> sm;
+    uint32_t unit;
+    int s;
+    while (next_unit(A, unit, s)) {
+        if (ab_bp::all_upright(A.scans[s])) ab_bp::bp_columns<RAYCAST, BILIN, 8>(A.scans[s], unit, sm);
+    }
     retire(A.g);
 }
 
 // Backprojection kernel variant code: ORD + 3 * mode (ORD from ab_bp::bp_ord),
 // mode 0 fast nearest, 1 fast bilinear, 2 raycast nearest, 3 raycast
-// bilinear, 4 exact; 15: fast nearest in the z-column layout (ORD 3) with 4
+// bilinear, 4 exact; 15: fast nearest in the z-lane layout (ORD 3) with 4
 // voxels per thread, 16: the same with 8 (every scan at least 256 voxels tall).
+// kCols is added where the scans may take the z columns.
+constexpr int kCols = 32;
 int bp_variant(const aprict_backproject_config *c, const aprict_vol_desc *vd) {
     const int mode = c->exact ? 4
                               : (c->approx_mode_direct_raycast ? 2 : 0) + (c->approx_mode_linear_interpolate ? 1 : 0);
@@ -169,38 +194,57 @@ int bp_variant(const aprict_backproject_config *c, const aprict_vol_desc *vd) {
 }
 
 // The batch backprojection kernel of a variant code.
-template <int V>
+template <int V, bool COLS>
 auto bp_kernel() {
     if constexpr (V == 16) {
-        return k_batch_backproject<3, false, false, false, 8>;
+        return k_batch_backproject<3, false, false, false, COLS, 8>;
     } else {
         constexpr int ORD = V == 15 ? 3 : V % 3, mode = V == 15 ? 0 : V / 3;
-        return k_batch_backproject<ORD, mode == 4, mode == 2 || mode == 3, mode == 1 || mode == 3>;
+        // one-layer volumes and the exact mode have no columns
+        return k_batch_backproject<ORD, mode == 4, mode == 2 || mode == 3, mode == 1 || mode == 3,
+                                   COLS && ORD != 2 && mode != 4>;
+    }
+}
+
+// The z-column kernel of a variant code's mode (15 and 16 are mode 0).
+template <class F>
+int with_columns_kernel(int variant, F &&f) {
+    const int v = variant & (kCols - 1);
+    switch (v < 15 ? v / 3 : 0) {
+        case 1: return f(k_batch_columns<false, true>);
+        case 2: return f(k_batch_columns<true, false>);
+        case 3: return f(k_batch_columns<true, true>);
+        default: return f(k_batch_columns<false, false>);
+    }
+}
+
+template <bool COLS, class F>
+int with_bp_kernel_of(int variant, F &&f) {
+    switch (variant) {
+        case 0: return f(bp_kernel<0, COLS>());
+        case 1: return f(bp_kernel<1, COLS>());
+        case 2: return f(bp_kernel<2, COLS>());
+        case 3: return f(bp_kernel<3, COLS>());
+        case 4: return f(bp_kernel<4, COLS>());
+        case 5: return f(bp_kernel<5, COLS>());
+        case 6: return f(bp_kernel<6, COLS>());
+        case 7: return f(bp_kernel<7, COLS>());
+        case 8: return f(bp_kernel<8, COLS>());
+        case 9: return f(bp_kernel<9, COLS>());
+        case 10: return f(bp_kernel<10, COLS>());
+        case 11: return f(bp_kernel<11, COLS>());
+        case 12: return f(bp_kernel<12, COLS>());
+        case 13: return f(bp_kernel<13, COLS>());
+        case 14: return f(bp_kernel<14, COLS>());
+        case 15: return f(bp_kernel<15, COLS>());
+        case 16: return f(bp_kernel<16, COLS>());
+        default: return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "corrupt batch plan (variant %d)", variant);
     }
 }
 
 template <class F>
 int with_bp_kernel(int variant, F &&f) {
-    switch (variant) {
-        case 0: return f(bp_kernel<0>());
-        case 1: return f(bp_kernel<1>());
-        case 2: return f(bp_kernel<2>());
-        case 3: return f(bp_kernel<3>());
-        case 4: return f(bp_kernel<4>());
-        case 5: return f(bp_kernel<5>());
-        case 6: return f(bp_kernel<6>());
-        case 7: return f(bp_kernel<7>());
-        case 8: return f(bp_kernel<8>());
-        case 9: return f(bp_kernel<9>());
-        case 10: return f(bp_kernel<10>());
-        case 11: return f(bp_kernel<11>());
-        case 12: return f(bp_kernel<12>());
-        case 13: return f(bp_kernel<13>());
-        case 14: return f(bp_kernel<14>());
-        case 15: return f(bp_kernel<15>());
-        case 16: return f(bp_kernel<16>());
-        default: return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "corrupt batch plan (variant %d)", variant);
-    }
+    return variant & kCols ? with_bp_kernel_of<true>(variant & (kCols - 1), f) : with_bp_kernel_of<false>(variant, f);
 }
 
 // Multiprocessor count of the current device, cached per device ordinal (a
@@ -234,10 +278,9 @@ int grid_for(K kernel, uint32_t n_units, int32_t &grid) {
 }
 
 template <class Params, class K>
-int launch_group(K kernel, const PlanHeader *H, const Group &gh, Group *gd, const char *params_host,
+int launch_group(K kernel, int grid, const Group &gh, Group *gd, const char *params_host,
                  cudaStream_t st) {
     if (gh.n_units == 0) return APRICT_OK;
-    const int grid = gh.grid;
     if (grid <= 0) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "corrupt batch plan (grid)");
     BatchArgs<Params> A;
     A.g = gd;
@@ -245,7 +288,6 @@ int launch_group(K kernel, const PlanHeader *H, const Group &gh, Group *gd, cons
     A.n_units = gh.n_units;
     memcpy(A.prefix, gh.prefix, sizeof(A.prefix));
     memcpy(A.scans, params_host + (size_t)gh.first * sizeof(Params), sizeof(Params) * gh.count);
-    (void)H;
     kernel<<<grid, 256, 0, st>>>(A);
     return ab_cuda_check(cudaGetLastError(), "batch launch");
 }
@@ -263,8 +305,8 @@ extern "C" size_t aprict_b200_batch_plan_bytes(int op, int n_scans) {
     return plan_bytes(op, n_scans);
 }
 
-extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_scans, const void *configs,
-                                      void *plan_host, size_t plan_capacity) {
+extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, int n_scans, const void *configs,
+                                            const uint32_t *views, void *plan_host, size_t plan_capacity) {
     if (op != APRICT_BATCH_PROJECT && op != APRICT_BATCH_BACKPROJECT)
         return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "unknown batch operation %d", op);
     if (scans == nullptr || configs == nullptr || plan_host == nullptr || n_scans <= 0)
@@ -283,7 +325,7 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
     std::vector<ab_bp::BPParams> bp(op == APRICT_BATCH_BACKPROJECT ? n_scans : 0);
     bool all_small = true, all_ss1 = true;
     int variant = -1;
-    // The z-column layout for a backprojection batch only when every scan
+    // The z-lane brick layout for a backprojection batch only when every scan
     // qualifies (one kernel variant per plan; each scan then gets the layout
     // its one-scan call would take).
     bool zlanes = op == APRICT_BATCH_BACKPROJECT && n_scans > 0;
@@ -295,6 +337,17 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
         tall = tall && scans[i].vol.nz >= 256u;
     }
     const bool zl8 = zlanes && tall && ab_tuning_get(AB_TUNE_BP_XB) == 0;
+    // The z-column kernel for a backprojection batch only when every scan may
+    // take it (one kernel variant per plan) and some scan's views allow it.
+    bool cols = op == APRICT_BATCH_BACKPROJECT, some = false;
+    for (int i = 0; cols && i < n_scans; ++i) {
+        cols = ab_bp::bp_columns_ok(&scans[i].vol, &scans[i].projs,
+                                    static_cast<const aprict_backproject_config *>(configs) + i);
+        if (views != nullptr && views[i] > APRICT_VIEWS_GENERAL)
+            return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "scan %d: unknown view promise %u", i, views[i]);
+        some = some || views == nullptr || views[i] != APRICT_VIEWS_GENERAL;
+    }
+    cols = cols && some;
     for (int i = 0; i < n_scans; ++i) {
         const aprict_scan &sc = scans[i];
         int rc;
@@ -312,14 +365,15 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
             units[i] = u;
         } else {
             const aprict_backproject_config *cfg = static_cast<const aprict_backproject_config *>(configs) + i;
-            int xb = 0, ord = -1;
-            uint64_t u = 0;
+            int xb = 0, ord = -1, cxb = 8;
+            uint64_t u = 0, cu = 0;
             rc = ab_bp::make_bp_params(sc.specs_dev, &sc.projs, sc.projs_dev, &sc.vol, sc.vol_dev, sc.multiplier_dev,
                                        cfg, sc.status_dev, bp[i], u, xb,
                                        zl8 ? 8 : batch_xb(ab_bp::bp_ord(&sc.vol), cfg->exact != 0),
-                                       zlanes ? &ord : nullptr);
+                                       zlanes ? &ord : nullptr, cols ? &cxb : nullptr, &cu);
             if (rc != APRICT_OK) return scan_error(rc, i);
-            const int v = ord == 3 ? (xb == 8 ? 16 : 15) : bp_variant(cfg, &sc.vol);
+            bp[i].views = views != nullptr ? (int)views[i] : (int)APRICT_VIEWS_UNKNOWN;
+            const int v = (ord == 3 ? (xb == 8 ? 16 : 15) : bp_variant(cfg, &sc.vol)) + (cols ? kCols : 0);
             if (variant >= 0 && v != variant)
                 return ab_fail(APRICT_ERR_INVALID_ARGUMENT,
                                "scan %d: every scan of a backprojection batch needs the same volume order, "
@@ -327,7 +381,7 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
                                "nearest / bilinear)",
                                i);
             variant = v;
-            units[i] = u;
+            units[i] = u > cu ? u : cu;  // the larger of the two kernels' (an order passes over units past its end)
         }
     }
     // projection variant: bit 0 = 64-bit offsets, bit 1 = sub-rays (ssu or ssv > 1)
@@ -372,6 +426,8 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
                 }
             } else {
                 rc = with_bp_kernel(variant, [&](auto k) { return grid_for(k, G->n_units, G->grid); });
+                if (rc == APRICT_OK && (variant & kCols))
+                    rc = with_columns_kernel(variant, [&](auto k) { return grid_for(k, G->n_units, G->col_grid); });
             }
         }
         if (rc != APRICT_OK) return rc;
@@ -389,6 +445,11 @@ extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_sc
         }
     }
     return APRICT_OK;
+}
+
+extern "C" int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_scans, const void *configs,
+                                      void *plan_host, size_t plan_capacity) {
+    return aprict_b200_batch_plan_views(op, scans, n_scans, configs, nullptr, plan_host, plan_capacity);
 }
 
 extern "C" int aprict_b200_batch_run(const void *plan_host, void *plan_dev, aprict_stream_t stream) {
@@ -411,16 +472,20 @@ extern "C" int aprict_b200_batch_run(const void *plan_host, void *plan_dev, apri
             using F32 = ab_fp::FPScan<int32_t>;
             using F64 = ab_fp::FPScan<int64_t>;
             switch (H->variant) {
-                case 0: rc = launch_group<F32>(k_batch_project<int32_t, true>, H, gh, gd, params, st); break;
-                case 1: rc = launch_group<F64>(k_batch_project<int64_t, true>, H, gh, gd, params, st); break;
-                case 2: rc = launch_group<F32>(k_batch_project<int32_t, false>, H, gh, gd, params, st); break;
-                case 3: rc = launch_group<F64>(k_batch_project<int64_t, false>, H, gh, gd, params, st); break;
+                case 0: rc = launch_group<F32>(k_batch_project<int32_t, true>, gh.grid, gh, gd, params, st); break;
+                case 1: rc = launch_group<F64>(k_batch_project<int64_t, true>, gh.grid, gh, gd, params, st); break;
+                case 2: rc = launch_group<F32>(k_batch_project<int32_t, false>, gh.grid, gh, gd, params, st); break;
+                case 3: rc = launch_group<F64>(k_batch_project<int64_t, false>, gh.grid, gh, gd, params, st); break;
                 default: return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "corrupt batch plan (variant %d)", H->variant);
             }
         } else {
-            rc = with_bp_kernel(H->variant, [&](auto k) {
-                return launch_group<ab_bp::BPParams>(k, H, gh, gd, params, st);
-            });
+            using P = ab_bp::BPParams;
+            rc = APRICT_OK;
+            if (H->variant & kCols)
+                rc = with_columns_kernel(H->variant,
+                                         [&](auto k) { return launch_group<P>(k, gh.col_grid, gh, gd, params, st); });
+            if (rc == APRICT_OK)
+                rc = with_bp_kernel(H->variant, [&](auto k) { return launch_group<P>(k, gh.grid, gh, gd, params, st); });
         }
         if (rc != APRICT_OK) return rc;
     }

@@ -35,6 +35,14 @@ constexpr int kThreads = 256;  // 32 (fast axis) x 8 (middle axis)
 template <int XB>
 constexpr int chunk_views() { return XB == 8 ? 64 : 128; }
 
+// Work-unit order: super-bricks, each all blocks of the fastest axis times a
+// compact group of the other two, about one wave of resident CTAs.
+struct BrickOrder {
+    int gb[3];     // blocks along fastest, middle, slowest axis
+    int sb1, sb2;  // super-brick extent in blocks along middle, slowest axis
+    int nsb1;      // super-bricks along the middle axis
+};
+
 struct BPParams {
     const aprict_proj_spec *specs;
     uint32_t n_views, nu, nv;
@@ -53,10 +61,12 @@ struct BPParams {
     float c0[3];     // volume centre (world)
     double cornerd[3];
     double vwd;
-    // brick-ordered CTA remap
-    int gb[3];       // blocks along fastest, middle, slowest axis
-    int sb1, sb2;    // super-brick extent in blocks along middle, slowest axis
-    int nsb1;        // super-bricks along the middle axis
+    BrickOrder brick;  // work-unit order of the bricks (bp_brick)
+    BrickOrder col;    // work-unit order of the z columns (bp_columns)
+    // Which views the caller promises (APRICT_VIEWS_*): with no promise, the
+    // z-column kernel and the brick kernel are both launched and each leaves
+    // when the views are the other's.
+    int views;
     // config
     int mask;
     float mask_r2;
@@ -250,6 +260,34 @@ __device__ __forceinline__ float zpow(const BPParams &P, const ab_bpview &b, flo
     return w;
 }
 
+// Whether scan P takes the z columns: by the caller's promise, else when every
+// view is upright, uniformly over the CTA (a barrier). With a weight in Z, Z
+// has to be constant along z too.
+__device__ __forceinline__ bool all_upright(const BPParams &P) {
+    if (P.views != (int)APRICT_VIEWS_UNKNOWN) return P.views == (int)APRICT_VIEWS_UPRIGHT;
+    const bool needZ = P.pL != 0 || P.pV != 0 || P.preset != 0;
+    bool tilted = false;
+    for (uint32_t v = threadIdx.x; v < P.n_views; v += kThreads) {
+        const aprict_proj_spec &sp = P.specs[v];
+        tilted = tilted || !(sp.det_u.z == 0.f && sp.det_v.x == 0.f && sp.det_v.y == 0.f) ||
+                 (needZ && sp.det_pos.z != sp.source_pos.z);
+    }
+    return !__syncthreads_or(tilted);
+}
+
+// Block coordinates of work unit `unit`; false past the volume (super-bricks
+// at its far edges).
+__device__ __forceinline__ bool brick_coords(const BrickOrder &O, uint32_t unit, int &b0, int &b1, int &b2) {
+    const int per_sb = O.gb[0] * O.sb1 * O.sb2;
+    const int sb = (int)unit / per_sb;
+    int r = (int)unit - sb * per_sb;
+    b0 = r % O.gb[0];
+    r /= O.gb[0];
+    b1 = (sb % O.nsb1) * O.sb1 + r % O.sb1;
+    b2 = (sb / O.nsb1) * O.sb2 + r / O.sb1;
+    return b1 < O.gb[1] && b2 < O.gb[2];
+}
+
 // EXACT: chord-length footprint (CB_backproject.cu:408-477).
 // RAYCAST: fast mode with direct-raycast weights (:512-646, preset 0).
 // BILIN: bilinear instead of nearest detector sampling.
@@ -275,15 +313,12 @@ static_assert(chunk_views<2>() <= 256 && chunk_views<2>() % 32 == 0 && chunk_vie
 // registers a thread, in the exact mode too.
 constexpr int kExactBlocks = 4;
 constexpr int bp_min_blocks(int xb, bool exact) { return exact ? kExactBlocks : (xb == 8 ? 3 : 4); }
+constexpr int kColBlocks = 4;  // the z-column kernels (ab_bpcol.cuh)
 // Default voxels per thread: 4 in the fast modes, 2 in the exact mode (whose
 // per-voxel footprint loop gains nothing from sharing a view's coefficients).
 constexpr int default_xb(bool exact) { return exact ? 2 : 4; }
 
-// Whether a kernel variant keeps the per-warp view table (the z-column
-// layout's fast nearest mode).
-constexpr bool bp_ztable(int ord, bool exact, bool raycast, bool bilin) { return ord == 3 && !exact && !raycast && !bilin; }
-
-template <bool EXACT, bool BILIN, int XB, bool ZT = false>
+template <bool EXACT, bool BILIN, int XB>
 struct BPSmem {
     static constexpr bool kNear = !EXACT && !BILIN;
     static constexpr int kQCap = 32 + 32 * XB;  // a flush leaves < 32; one view adds <= 32 * XB
@@ -297,15 +332,10 @@ struct BPSmem {
     uint8_t inner[kChunk];    // per view: every voxel of the CTA projects into the flat box
     int vcount;               // views of the chunk whose brick projection reaches the detector
     uint8_t off_det[kChunk];  // per view: the whole brick projects beyond one detector edge
-    uint8_t zinv[kChunk];     // per view: depth and u do not change along z (ORD 3 shares them)
+    uint8_t zinv[kChunk];     // per view: depth and u do not change along z (the exact mode's ORD 3 shares them)
     uint8_t vzero[kChunk];    // per view (slice stacks): one detector row, v form identically zero
     uint8_t vlist[kChunk];    // those views' indices in the chunk, in order
     uint16_t q[EXACT ? 1 : kWarps][EXACT ? 1 : kQCap];
-    // Nearest mode, z-column layout: per warp, the warp-uniform part of 32
-    // consecutive views of the chunk (rD, weight, and the 64-bit byte address
-    // of the column's pixel 0 less 4 * 0x4B400000 * sv, split in two words; rD
-    // NaN when the warp's column misses the detector)
-    float4 zrec[ZT ? kWarps : 1][ZT ? 32 : 1];
     // Compensated per-voxel totals over the view chunks: sum and Kahan term,
     // [warp][lane * XB + k], each slot owned by one thread.
     float ksum[kWarps][32 * XB];
@@ -317,7 +347,7 @@ struct BPSmem {
 // __syncthreads and returns uniformly.
 template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, int XB, bool SKIP = RAYCAST>
 __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
-                                         BPSmem<EXACT, BILIN, XB, bp_ztable(ORD, EXACT, RAYCAST, BILIN)> &sm) {
+                                         BPSmem<EXACT, BILIN, XB> &sm) {
     static_assert(XB == 2 || XB == 4 || XB == 8, "XB is 2, 4 or 8");
     constexpr int kXB = XB, kKB = q_kbits<XB>();
     constexpr int kChunk = chunk_views<XB>();
@@ -327,14 +357,8 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
     ab_bpview_exact *sx = sm.sx;
 
     // Brick-ordered block coordinates (uniform per CTA).
-    const int per_sb = P.gb[0] * P.sb1 * P.sb2;
-    const int sb = (int)brick / per_sb;
-    int r = (int)brick - sb * per_sb;
-    const int b0 = r % P.gb[0];
-    r /= P.gb[0];
-    const int b1 = (sb % P.nsb1) * P.sb1 + r % P.sb1;
-    const int b2 = (sb / P.nsb1) * P.sb2 + r / P.sb1;
-    if (b1 >= P.gb[1] || b2 >= P.gb[2]) return;  // the whole CTA returns before any barrier
+    int b0, b1, b2;
+    if (!brick_coords(P.brick, brick, b0, b1, b2)) return;  // the whole CTA returns before any barrier
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // Axes: a0 along the lanes (memory-contiguous), a1 along the warps, a2
@@ -342,11 +366,9 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
     // (x, y, z); ORD 2: C order with nz == 1 (slices): lanes along y (stride
     // 1), warps and XB both along x, z = 0. ORD 3: C order with the lanes and
     // each thread's XB voxels all along z (voxel k of a lane 32 k further),
-    // one x layer per CTA: a thread's voxels then share x and y, so for views
-    // whose detector u axis and normal have no z component (circular and
-    // helical scans with an upright detector) the voxels share their depth and
-    // u coordinate, which are computed once per warp and view (the fast modes)
-    // or once per thread and view (the exact mode).
+    // one x layer per CTA: a thread's voxels then share x and y, and in the
+    // exact mode, for upright detectors, their depth and u coordinates (upright
+    // views in the fast modes take ab_bpcol.cuh).
     constexpr bool kZ = ORD == 3;
     constexpr int a0 = ORD == 0 || ORD == 3 ? 2 : (ORD == 1 ? 0 : 1);
     constexpr int a1 = ORD == 2 ? 2 : 1;
@@ -578,15 +600,12 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
                                                (a2 == 0 ? bt.nv.x : (a2 == 1 ? bt.nv.y : bt.nv.z)) * vws,
                                                (a2 == 0 ? bt.den.x : (a2 == 1 ? bt.den.y : bt.den.z)) * vws,
                                                (a2 == 0 ? bt.zl.x : (a2 == 1 ? bt.zl.y : bt.zl.z)) * vws);
-                        // exact zeros in the z coefficients, FP32 and FP64 alike (ORD 3 only)
-                        if constexpr (EXACT)  // and the detector's v axis has no x-y component
+                        // exact zeros in the z coefficients (ORD 3), and the detector's v axis
+                        // has no x-y component
+                        if constexpr (EXACT)
                             sm.zinv[t] = (uint8_t)(kZ && bt.den.z == 0.f && bt.nu.z == 0.f &&
                                                    (!needZ || bt.zl.z == 0.f) && sx[t].v.x == 0.f &&
                                                    sx[t].v.y == 0.f);
-                        else
-                            sm.zinv[t] = (uint8_t)(kZ && kNear && bt.den.z == 0.f && bt.nu.z == 0.f &&
-                                                   (!needZ || bt.zl.z == 0.f) && svd[t].nu[2] == 0.0 &&
-                                                   svd[t].den[2] == 0.0);
                         // A fan-beam slice: the v form vanishes in the slice plane (its x, y
                         // and constant coefficients are exact zeros), and with one z layer
                         // and no z sub-samples every sample lies in that plane (z = 0
@@ -618,50 +637,6 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
                     if (!__any_sync(0xffffffffu, any_live)) continue;
                     const int n_list = kSkip ? sm.vcount : cn;
                     for (int j = 0; j < n_list; ++j) {
-                        if constexpr (kZ && kNear && !RAYCAST) {
-                            if ((j & 31) == 0) {
-                                // The warp's table for views j .. j + 31: every lane of
-                                // the warp has this x and y, so for a view whose depth and
-                                // u coordinate do not change along z (zinv) everything
-                                // that depends on u is warp-uniform -- the reciprocal
-                                // depth, the weight, the u half of the pixel choice (FP64
-                                // for a near tie), the u half of the edge taper and
-                                // whether the column lies on the detector. Lane L settles
-                                // view j + L once for the warp's 32 x XB voxels.
-                                const int jj = j + lane;
-                                const int tt = jj < n_list ? (kSkip ? (int)sm.vlist[jj] : jj) : 0;
-                                if (jj < n_list && sm.zinv[tt]) {
-                                    const ab_bpview bq = sv[tt];
-                                    const float rDq = rcp_fast(dot4(bq.den, X0, Y0, Z0));
-                                    const float fu = dot4(bq.nu, X0, Y0, Z0) * rDq;
-                                    float w = rDq * rDq;
-                                    if (needZ) w *= zpow(P, bq, dot4(bq.zl, X0, Y0, Z0));
-                                    float du;
-                                    int iu = round_index(fu, -2.f, P.fnu1, du);
-                                    if (fabsf(du) > bq.tie_u) {
-                                        const VoxRef vr{((double)b2 + 0.5 + (double)fsub[0] - 0.5 * P.n[0]) * P.vwd,
-                                                        ((double)i1 + 0.5 + (double)fsub[1] - 0.5 * P.n[1]) * P.vwd,
-                                                        0.0};
-                                        iu = refine_index(svd[tt].nu, svd[tt].den, vr, iu, du);
-                                    }
-                                    float4 rec = make_float4(__int_as_float(0x7fc00000), 0.f, 0.f, 0.f);
-                                    if ((unsigned)iu < P.nu) {
-                                        const float cu = fu - bq.cu0;
-                                        if (P.sep > 0.f && fabsf(cu) > bq.tap_ru)
-                                            w *= ab_edge_taper_half(fabsf(cu), bq.inv_halfu, P.inv_sep);
-                                        // + 4 sv bits(tv) is then the byte address of row round(fv)
-                                        const uint64_t col =
-                                            (uint64_t)(uintptr_t)(P.projs + (int64_t)(v0 + tt) * P.stride_view +
-                                                                  (int64_t)iu * P.su) -
-                                            4ull * 0x4B400000ull * (uint64_t)(uint32_t)P.sv;
-                                        rec = make_float4(rDq, w, __uint_as_float((uint32_t)col),
-                                                          __uint_as_float((uint32_t)(col >> 32)));
-                                    }
-                                    sm.zrec[warp][lane] = rec;
-                                }
-                                __syncwarp();
-                            }
-                        }
                         const int t = kSkip ? (int)sm.vlist[j] : j;
                         const int view = (int)v0 + t;
                         const ab_bpview b = sv[t];
@@ -873,71 +848,7 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
                             // detector-edge taper band) are flagged and finished in a rare
                             // second pass, so the common path has no divergent branches.
                             unsigned pending = 0;
-                            // ORD 3 on a view whose depth, u coordinate and distance along
-                            // the axis do not change along z (exact zeros in the per-view
-                            // steps; warp-uniform): the thread's voxels share rD, fu, the
-                            // weight and the u half of the pixel choice, computed once.
-                            const bool zinv = kZ && kNear && !RAYCAST && sm.zinv[t];
-                            if (zinv) {
-                                // the warp-uniform part from the warp's table (filled above)
-                                const float4 rec = sm.zrec[warp][j & 31];
-                                const float rD = rec.x;
-                                if (rD == rD) {  // else the column is off the detector: zeros
-                                    const float w = rec.y;
-                                    const uint64_t col = ((uint64_t)__float_as_uint(rec.w) << 32) | __float_as_uint(rec.z);
-                                    const uint32_t sv4 = 4u * (uint32_t)P.sv;
-                                    // Interior column: fv is monotone in k, so when the first and
-                                    // last voxel of every lane lie in the flat box, all of the
-                                    // warp's rows are on the detector with taper weight 1 and only
-                                    // a near-tie row choice remains. That pass has no predicates:
-                                    // it loads every voxel's FP32-rounded pixel (live or not; dead
-                                    // voxels are never written) and turns the tie test into an
-                                    // FMA-pipe value slow = 0 or 1 that zeroes the weight and sets
-                                    // the voxel's bit of the fix-up mask.
-                                    const float fvf = fmaf(0.f, dNv, Nv0) * rD;
-                                    const float fvl = fmaf((float)(kXB - 1), dNv, Nv0) * rD;
-                                    const bool inbox = fabsf(fvf - b.cv0) <= b.tap_rv && fabsf(fvl - b.cv0) <= b.tap_rv;
-                                    if (__all_sync(0xffffffffu, inbox) && b.tie_v >= 0.25f) {
-                                        // |dv| and tie_v lie in [0, 1/2] and tie_v >= 1/4: |dv| > tie_v
-                                        // means |dv| - tie_v >= 2^-25, so 2^40 (|dv| - tie_v)
-                                        // saturates to exactly 1, and to 0 otherwise
-                                        const float ntie = -b.tie_v * 0x1p40f;
-                                        float pendf = 0.f;
-#pragma unroll
-                                        for (int k = 0; k < kXB; ++k) {
-                                            const float fv = fmaf((float)k, dNv, Nv0) * rD;
-                                            const float tv = __fadd_rn(fv, kMagic);
-                                            const float dv = __fsub_rn(fv, __fsub_rn(tv, kMagic));
-                                            const float slow = __saturatef(fmaf(fabsf(dv), 0x1p40f, ntie));
-                                            const float pv = __ldg(reinterpret_cast<const float *>(
-                                                col + (uint64_t)(uint32_t)__float_as_int(tv) * sv4));
-                                            acc[k] = fmaf(pvp[k], wp[k], acc[k]);
-                                            pvp[k] = pv;
-                                            wp[k] = fmaf(-slow, w, w);
-                                            pendf = fmaf(slow, (float)(1u << k), pendf);
-                                        }
-                                        pending = (unsigned)pendf;
-                                    } else {
-#pragma unroll
-                                    for (int k = 0; k < kXB; ++k) {
-                                        const float fv = fmaf((float)k, dNv, Nv0) * rD;
-                                        const float av = fabsf(fv - b.cv0);
-                                        const bool outside = kSkip && av > b.out_rv;
-                                        const float tv = __fadd_rn(fv, kMagic);
-                                        const float dv = __fsub_rn(fv, __fsub_rn(tv, kMagic));
-                                        const bool fast = av <= b.tap_rv && fabsf(dv) <= b.tie_v;
-                                        float pv = 0.f;
-                                        if (live[k] && fast)
-                                            pv = __ldg(reinterpret_cast<const float *>(
-                                                col + (uint64_t)(uint32_t)__float_as_int(tv) * sv4));
-                                        acc[k] = fmaf(pvp[k], wp[k], acc[k]);
-                                        pvp[k] = pv;
-                                        wp[k] = w;
-                                        pending |= (live[k] && !fast && !outside) ? 1u << k : 0u;
-                                    }
-                                    }
-                                }
-                            } else if (ORD == 2 && !BILIN && sm.vzero[t]) {
+                            if (ORD == 2 && !BILIN && sm.vzero[t]) {
                                 // Fan-beam slice: one detector row and a v form that is zero
                                 // at every point, so every voxel projects onto row 0 exactly
                                 // (v = 0 = the row centre, no tie, inside the flat box in v);
@@ -1180,11 +1091,10 @@ inline int bp_ord(const aprict_vol_desc *vd) { return vd->order == 0 ? (vd->nz =
 // Host: whether ORD 3 (lanes and a thread's voxels along z) applies: the
 // fast nearest mode, or the exact mode where exact_ok (one-scan calls), on a
 // C-order volume tall enough to fill the 32 XB voxels of a thread column,
-// unless tuning knob 7 is 1, with a v stride below 2^30 elements (the gathers
-// form their byte address as a 32 x 32-bit product). Measured on a 256^3
-// volume with 360 views: nearest 9.82 -> 8.68 ms; on 128^3 with 180 views,
-// exact 10.0 -> 7.1 ms (the column's x-y quantities shared); bilinear (27.4 vs
-// 28.1 ms) keeps ORD 0.
+// unless tuning knob 7 is 1, with a v stride below 2^30 elements. Measured on
+// 128^3 with 180 views, exact: 10.0 -> 7.1 ms (the column's x-y quantities
+// shared); nearest with tilted detectors, 256^3 x 360 views: 8.7 -> 7.5 ms;
+// bilinear (27.4 vs 28.1 ms) keeps ORD 0.
 inline bool bp_zlanes_ok(const aprict_vol_desc *vd, const aprict_proj_desc *pd, int xb,
                          const aprict_backproject_config *cfg, bool exact_ok = false) {
     return bp_ord(vd) == 0 && ab_tuning_get(AB_TUNE_BP_ZLANES) != 1 && vd->nz >= 32u * (uint32_t)xb &&
@@ -1192,15 +1102,59 @@ inline bool bp_zlanes_ok(const aprict_vol_desc *vd, const aprict_proj_desc *pd, 
            !cfg->approx_mode_linear_interpolate;
 }
 
+// Host: whether a call may take the z-column kernel (ab_bpcol.cuh) when its
+// views turn out to be upright: the fast modes on a volume of more than one
+// layer, unless tuning knob 7 is 1; nearest with a v stride below 2^30
+// elements (the gathers form their byte address as a 32 x 32-bit product),
+// bilinear with v contiguous (its row pairs are gathered at one address).
+inline bool bp_columns_ok(const aprict_vol_desc *vd, const aprict_proj_desc *pd, const aprict_backproject_config *cfg) {
+    return vd->nz > 1u && ab_tuning_get(AB_TUNE_BP_ZLANES) != 1 && !cfg->exact &&
+           (cfg->approx_mode_linear_interpolate ? pd->stride_v == 1 && pd->stride_u < (int64_t)1 << 30
+                                                : pd->stride_v < (int64_t)1 << 30);
+}
+
+// Voxels per thread of the z-column kernel: the fewest that hold the column
+// (blocks of 32 voxels past the volume's top are skipped, but the per-view
+// work of a warp is spread over its live blocks only).
+inline int col_xb(uint32_t nz) { return nz > 128u ? 8 : (nz > 64u ? 4 : 2); }
+
+// Host: super-bricks of about one wave of `resident` CTAs per SM, with equal
+// extents in voxels along the middle (8 per block) and slowest (ext2) axes;
+// false when the units overflow a grid.
+inline bool order_bricks(BrickOrder &O, int ext2, int resident, uint64_t &units) {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    }
+    const int wave = ab_tuning_get(AB_TUNE_BP_WAVE) > 0 ? ab_tuning_get(AB_TUNE_BP_WAVE) : resident;
+    const double target = (double)wave * sms / (double)O.gb[0];  // blocks of the (middle x slowest) plane per wave
+    int sb1 = (int)floor(sqrt(target * ext2 / 8.0) + 0.5);
+    sb1 = sb1 < 1 ? 1 : (sb1 > O.gb[1] ? O.gb[1] : sb1);
+    int sb2 = (int)floor(target / sb1 + 0.5);
+    sb2 = sb2 < 1 ? 1 : (sb2 > O.gb[2] ? O.gb[2] : sb2);
+    O.sb1 = sb1;
+    O.sb2 = sb2;
+    O.nsb1 = (O.gb[1] + sb1 - 1) / sb1;
+    const int64_t nsb = (int64_t)O.nsb1 * ((O.gb[2] + sb2 - 1) / sb2);
+    const int64_t grid = nsb * O.gb[0] * sb1 * sb2;
+    units = (uint64_t)grid;
+    return grid <= 0x7fffffffLL;
+}
+
 // Host: validate one backprojection call and fill its parameters; units is
 // the number of work units (bricks, 0 when empty), xb the voxels per thread
 // (force_xb 2, 4 or 8, or 0 for the tuning knob's choice). With ord_out the
 // caller accepts ORD 3 where bp_zlanes_ok holds and learns the layout chosen;
-// without it the layout is bp_ord's.
+// without it the layout is bp_ord's. cxb: the z-column kernel's voxels per
+// thread where it may run (in: a choice, or 0; out: 0 where it may not), with
+// col_units work units.
 inline int make_bp_params(const aprict_proj_spec *specs_dev, const aprict_proj_desc *pd, const float *projs_dev,
                           const aprict_vol_desc *vd, float *vol_dev, const float *multiplier_dev,
                           const aprict_backproject_config *cfg, uint32_t *status_dev, BPParams &P,
-                          uint64_t &units, int &xb, int force_xb = 0, int *ord_out = nullptr) {
+                          uint64_t &units, int &xb, int force_xb = 0, int *ord_out = nullptr, int *cxb = nullptr,
+                          uint64_t *col_units = nullptr) {
     units = 0;
     int rc;
     if ((rc = ab_check_projs(pd, projs_dev, "projections")) != APRICT_OK) return rc;
@@ -1282,48 +1236,37 @@ inline int make_bp_params(const aprict_proj_spec *specs_dev, const aprict_proj_d
     xb = forced ? force_xb : (knob == 2 || knob == 4 || knob == 8 ? knob : default_xb(cfg->exact != 0));
     const int ord = ord_out && bp_zlanes_ok(vd, pd, xb, cfg, true) ? 3 : bp_ord(vd);
     if (ord_out) *ord_out = ord;
-    // z columns of 8 voxels per thread where the volume is tall enough (the
-    // per-view work of a thread is shared by twice as many voxels: sirt256
-    // 8.66 -> 8.35 ms), unless the caller or the knob chose
+    // 8 voxels per thread where the volume is tall enough (the per-view work
+    // of a thread is shared by twice as many voxels), unless the caller or the
+    // knob chose
     if (ord == 3 && !forced && knob == 0 && vd->nz >= 256u && !cfg->exact) xb = 8;
     const int kXB = xb;
+    BrickOrder &O = P.brick;
     if (ord == 2) {  // slices: lanes along y, warps x XB along x
-        P.gb[0] = (P.n[1] + 31) / 32;
-        P.gb[1] = (P.n[0] + 8 * kXB - 1) / (8 * kXB);
-        P.gb[2] = 1;
+        O.gb[0] = (P.n[1] + 31) / 32;
+        O.gb[1] = (P.n[0] + 8 * kXB - 1) / (8 * kXB);
+        O.gb[2] = 1;
     } else if (ord == 3) {  // z columns of 32 XB voxels, warps along y, one x layer
-        P.gb[0] = (P.n[2] + 32 * kXB - 1) / (32 * kXB);
-        P.gb[1] = (P.n[1] + 7) / 8;
-        P.gb[2] = P.n[0];
+        O.gb[0] = (P.n[2] + 32 * kXB - 1) / (32 * kXB);
+        O.gb[1] = (P.n[1] + 7) / 8;
+        O.gb[2] = P.n[0];
     } else {
         const int n0 = ord == 0 ? P.n[2] : P.n[0], n1 = P.n[1], n2 = ord == 0 ? P.n[0] : P.n[2];
-        P.gb[0] = (n0 + 31) / 32;
-        P.gb[1] = (n1 + 7) / 8;
-        P.gb[2] = (n2 + kXB - 1) / kXB;
+        O.gb[0] = (n0 + 31) / 32;
+        O.gb[1] = (n1 + 7) / 8;
+        O.gb[2] = (n2 + kXB - 1) / kXB;
     }
-    // Super-brick: all blocks of the fastest axis x sb1 x sb2 blocks (8 and
-    // kXB voxels each; 8 and 1 for ORD 3), about one wave of resident CTAs,
-    // with equal extents in voxels along the middle and slowest axes.
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    bool fits = order_bricks(O, ord == 3 ? 1 : kXB, bp_min_blocks(xb, cfg->exact != 0), units);
+    if (cxb && bp_columns_ok(vd, pd, cfg)) {
+        if (*cxb == 0) *cxb = knob == 2 || knob == 4 || knob == 8 ? knob : col_xb(vd->nz);
+        P.col.gb[0] = (P.n[2] + 32 * *cxb - 1) / (32 * *cxb);
+        P.col.gb[1] = (P.n[1] + 7) / 8;
+        P.col.gb[2] = P.n[0];
+        fits = order_bricks(P.col, 1, kColBlocks, *col_units) && fits;
+    } else if (cxb) {
+        *cxb = 0;
     }
-    const int wave = ab_tuning_get(AB_TUNE_BP_WAVE) > 0 ? ab_tuning_get(AB_TUNE_BP_WAVE) : bp_min_blocks(xb, cfg->exact != 0);
-    const double target = (double)wave * sms / (double)P.gb[0];  // blocks of the (middle x slowest) plane per wave
-    const int ext2 = ord == 3 ? 1 : kXB;  // voxels of a block along the slowest axis
-    int sb1 = (int)floor(sqrt(target * ext2 / 8.0) + 0.5);
-    sb1 = sb1 < 1 ? 1 : (sb1 > P.gb[1] ? P.gb[1] : sb1);
-    int sb2 = (int)floor(target / sb1 + 0.5);
-    sb2 = sb2 < 1 ? 1 : (sb2 > P.gb[2] ? P.gb[2] : sb2);
-    P.sb1 = sb1;
-    P.sb2 = sb2;
-    P.nsb1 = (P.gb[1] + sb1 - 1) / sb1;
-    const int64_t nsb = (int64_t)P.nsb1 * ((P.gb[2] + sb2 - 1) / sb2);
-    const int64_t grid = nsb * P.gb[0] * sb1 * sb2;
-    if (grid > 0x7fffffffLL) return ab_fail(APRICT_ERR_TOO_LARGE, "volume too large for the grid");
-    units = (uint64_t)grid;
+    if (!fits) return ab_fail(APRICT_ERR_TOO_LARGE, "volume too large for the grid");
     return APRICT_OK;
 }
 

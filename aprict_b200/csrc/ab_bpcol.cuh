@@ -1,0 +1,424 @@
+// ab_bpcol.cuh -- voxel-driven backprojection of upright-detector views into
+// C-order volumes, one z column of the volume per warp.
+//
+// A view is upright when its detector's u axis and normal have no z component
+// (every circular, helical and cylindrical scan whose detector columns run
+// along z; an exact test on the FP32 view record). The voxels of a z column
+// then share their depth, their u coordinate and everything made from them,
+// and v is linear in z:
+//     f(n) = A + n S,   n = voxel index within the column.
+// Each warp owns one column of 32 XB voxels (lane l has voxels l + 32 k) and
+// works from a table of 32 views at a time, filled by one lane per view in
+// FP64: A and S (rounded once to FP32, relative to the centre row), the
+// weight with the u half of the detector-edge taper, the byte address of the
+// pixel column, the trust threshold of the row choice, and for each block of
+// 32 voxels whether it lies inside the detector's flat box, across its edge
+// or off the detector. A voxel-view inside the flat box then costs an fma, the
+// magic rounding, the tie test, one address multiply-add, the gather and one
+// fma; the arithmetic runs on pairs of voxels (fma.rn.f32x2).
+//
+// Row choice: A and S come from FP64, so the FP32 row coordinate is off by at
+// most u (2 |A| + 2 |n S| + |f|), u = 2^-24, some 5e-5 pixel on a 384-row
+// detector (ten times less than with forms rounded before the division). A
+// row whose fraction comes that close to 1/2 is decided again in FP64; such a
+// voxel-view occurs in about 2 % of the warp's views, so it is settled at
+// once, the difference to the pixel already gathered going to the voxel's
+// compensated total.
+//
+// Bound: gather latency and issue (on 256^3 x 360 views x 384^2 nearest: 12.5
+// warp instructions per 32 voxel-views against 21 of the brick kernel's z-lane
+// path before it, issue 54 %, L1 wavefronts 60 %). Measured there, four CTAs per
+// SM: nearest 4.93 -> 3.11 ms (F order 14.8 -> 3.3 ms: its lanes gathered 32
+// pixel columns), direct raycast 13.8 -> 3.1 ms, on a helical scan 12.4 -> 6.5 ms
+// (columns cut by the detector's edges); 64^3 x 90 views 72 -> 55 us; bilinear
+// on 210 x 190 x 150 x 200 views 2.06 -> 1.73 ms. Three CTAs at 80 registers, no
+// spills: 3.6 ms. Blocks across the detector's edge are gathered under a
+// predicate (a branch around the gather: 7.6 ms on the helical scan).
+#pragma once
+
+#include "ab_bpbrick.cuh"
+#include "ab_f32x2.cuh"
+
+namespace ab_bp {
+
+// One view as the column table is filled from it: the FP64 forms of
+// ab_bpview_d and the direct-raycast weights' inputs.
+struct ColView {
+    ab_bpview_d d;    // N_u, N_v, D of the position relative to the volume centre
+    float zl[3];      // Z = zl[0] x + zl[1] y + zl[2]: distance along the source-detector axis
+    float invL;
+    float kfast;      // voxwid^3 Dn^2 / (|u||v|): fast-mode weight kfast / D^2
+    float sxw, syw;   // source x, y (presets)
+    int ok;  // 0: a degenerate view, which adds nothing
+    float pad[2];
+};
+static_assert(sizeof(ColView) % 16 == 8, "an odd number of 8-byte words: 32 lanes read 32 records without bank conflicts");
+
+struct ColRec {
+    float4 a;  // A, S, weight, trust threshold of |f - round(f)|
+    uint4 b;   // column address (lo, hi), masks (inside | across << 8), unused
+};
+
+constexpr int kColWarps = kThreads / 32;
+
+template <int XB>
+struct ColSmem {
+    static constexpr int kChunk = 64;
+    ColView view[kChunk];
+    ColRec rec[kColWarps][32];
+    float ksum[kColWarps][32 * XB];   // compensated totals over the view chunks
+    float kcomp[kColWarps][32 * XB];
+};
+
+// ab_derive_bpview's FP64 forms for an upright view, by the same expressions
+// with the vanishing terms left out (the same values, a third of the work);
+// false for a degenerate view.
+__device__ __forceinline__ bool derive_upright(const aprict_proj_spec &sp, ab_d3 c0, ab_bpview_d &o, double &Dn, double &uu,
+                                               double &vv, ab_d3 &Ps, ab_d3 &c0s) {
+    const ab_d3 s = ab_d3_of(sp.source_pos), P = ab_d3_of(sp.det_pos);
+    const double ux = (double)sp.det_u.x, uy = (double)sp.det_u.y, vz = (double)sp.det_v.z;
+    const double nx = uy * vz, ny = -(ux * vz);
+    uu = ux * ux + uy * uy;
+    vv = vz * vz;
+    Ps = P - s;
+    c0s = c0 - s;
+    Dn = Ps.x * nx + Ps.y * ny;
+    o = ab_bpview_d{};
+    if (!(uu > 0.0 && vv > 0.0 && Dn != 0.0 && ab_finite3(s) && ab_finite3(P) && isfinite(uu) && isfinite(vv))) return false;
+    const double hu = ((double)sp.nu - 1.0) * 0.5, hv = ((double)sp.nv - 1.0) * 0.5;
+    const double q = ux * Ps.x + uy * Ps.y, iu = 1.0 / uu, iv = 1.0 / vv;
+    o.nu[0] = (ux * Dn - nx * q) * iu + nx * hu;
+    o.nu[1] = (uy * Dn - ny * q) * iu + ny * hu;
+    o.nu[3] = o.nu[0] * c0s.x + o.nu[1] * c0s.y;
+    const double r = vz * Ps.z;
+    o.nv[0] = -(nx * r) * iv + nx * hv;
+    o.nv[1] = -(ny * r) * iv + ny * hv;
+    o.nv[2] = vz * Dn * iv;
+    o.nv[3] = o.nv[0] * c0s.x + o.nv[1] * c0s.y + o.nv[2] * c0s.z;
+    o.den[0] = nx;
+    o.den[1] = ny;
+    o.den[3] = nx * c0s.x + ny * c0s.y;
+    return true;
+}
+
+// A gather when `on`, else 0, without a branch.
+__device__ __forceinline__ float ldg_if(uint64_t addr, bool on) {
+    float v;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"
+        : "=f"(v)
+        : "l"(addr), "r"((unsigned)on));
+    return v;
+}
+
+// The pixel of the row that holds f, decided in FP64 (0 off the detector). A
+// call: rare, and its FP64 temporaries stay out of the voxel loop's registers.
+static __device__ __noinline__ float col_exact_row(const ab_bpview_d &d, double X, double Y, double Z, float f, int crow, int nv,
+                                            uint64_t col, uint32_t sv4) {
+    const float t = __fadd_rn(f, kMagic);
+    const int i = __float_as_int(t) - 0x4B400000 + crow;
+    const int e = refine_index(d.nv, d.den, VoxRef{X, Y, Z}, i, __fsub_rn(f, __fsub_rn(t, kMagic)));
+    return (unsigned)e < (unsigned)nv
+               ? __ldg(reinterpret_cast<const float *>(col + (uint64_t)(uint32_t)(e - crow + 0x4B400000) * sv4))
+               : 0.f;
+}
+
+// Backprojects scan P, all of whose views are upright, into the columns of work unit
+// `brick` (in P.col's order). Every thread of the CTA calls it.
+// BILIN (v stride 1): two pixel columns and the weight between them in the
+// record, rows floor(f) and floor(f) + 1 of both gathered, and blended in
+// fetch_bilinear's order.
+template <bool RAYCAST, bool BILIN, int XB>
+__device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, ColSmem<XB> &sm) {
+    static_assert(XB % 2 == 0 && XB <= 8, "pairs of voxels, 8-bit block masks");
+    constexpr int kChunk = ColSmem<XB>::kChunk;
+    constexpr unsigned kAll = (1u << XB) - 1u;
+    int b0, b1, b2;
+    if (!brick_coords(P.col, brick, b0, b1, b2)) return;  // the whole CTA
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ix = b2, iy = b1 * 8 + warp, z0 = b0 * 32 * XB;
+    const float vw = P.voxwid;
+    bool col_live = iy < P.n[1];
+    if (col_live && P.mask) {  // the cylinder mask is the column's (about world x = y = 0)
+        const float xw = ((float)ix + 0.5f - 0.5f * (float)P.n[0]) * vw + P.c0[0];
+        const float yw = ((float)iy + 0.5f - 0.5f * (float)P.n[1]) * vw + P.c0[1];
+        col_live = !(xw * xw + yw * yw > P.mask_r2);
+    }
+    // live blocks of 32 voxels, and the pairs that hold them (a pair's dead
+    // block is gathered along when it lies on the detector, never written)
+    const int nb = min(XB, (P.n[2] - z0 + 31) / 32);
+    const unsigned blocks = (1u << nb) - 1u, pairs = (1u << ((nb + 1) & ~1)) - 1u;
+
+    float *ksum = sm.ksum[warp], *kcomp = sm.kcomp[warp];
+#pragma unroll
+    for (int k = 0; k < XB; ++k) ksum[lane + 32 * k] = kcomp[lane + 32 * k] = 0.f;
+
+    const int crow = (int)(P.nv >> 1);                                   // the centre row
+    const float coff = 0.5f * ((float)P.nv - 1.f) - (float)crow;        // detector centre relative to it
+    const float halfv = 0.5f * (float)P.nv;
+    const float inv_halfv = 2.f / (float)P.nv;
+    const float flatv = P.sep > 0.f ? halfv * ((1.f - P.sep) * (1.f - 1e-5f)) : halfv;
+    const float insidev = BILIN ? fminf(flatv, halfv - 0.5f) : flatv;  // both taps' rows on the detector
+    const float offv = BILIN ? halfv + 0.5f : halfv;
+    // (bilinear: v stride 1, kept a run-time factor so that the addresses are multiply-adds)
+    const uint32_t sv4 = 4u * (uint32_t)P.sv, su4 = 4u * (uint32_t)P.su;
+    const bool needZ = P.pL != 0 || P.pV != 0 || (RAYCAST && P.preset != 0);
+    const int n_sub = P.ssx * P.ssy * P.ssz;
+    const f32x2 magic = pk(kMagic, kMagic), nmagic = pk(-kMagic, -kMagic), minus1 = pk(-1.f, -1.f);
+    const f32x2 one = pk(1.f, 1.f), mhalf = pk(-0.5f, -0.5f);
+
+    for (int isub = 0; isub < n_sub; ++isub) {
+        const double fx = -0.5 + (0.5 + isub / (P.ssy * P.ssz)) / P.ssx;
+        const double fy = -0.5 + (0.5 + (isub / P.ssz) % P.ssy) / P.ssy;
+        const double fz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
+        // the column's first voxel relative to the volume centre
+        const double X = (ix + 0.5 + fx - 0.5 * P.n[0]) * P.vwd, Y = (iy + 0.5 + fy - 0.5 * P.n[1]) * P.vwd;
+        const double Z0 = (z0 + 0.5 + fz - 0.5 * P.n[2]) * P.vwd;
+        for (uint32_t v0 = 0; v0 < P.n_views; v0 += kChunk) {
+            const int cn = (int)min((uint32_t)kChunk, P.n_views - v0);
+            __syncthreads();
+            if ((int)threadIdx.x < cn) {
+                const ab_d3 c0d{P.cornerd[0] + 0.5 * P.vwd * P.n[0], P.cornerd[1] + 0.5 * P.vwd * P.n[1],
+                                P.cornerd[2] + 0.5 * P.vwd * P.n[2]};
+                const aprict_proj_spec sp = P.specs[v0 + threadIdx.x];
+                ColView &cv = sm.view[threadIdx.x];
+                double Dn, uu, vv;
+                ab_d3 Ps, c0s;
+                cv.ok = derive_upright(sp, c0d, cv.d, Dn, uu, vv, Ps, c0s);
+                if (!cv.ok && P.status) atomicOr(P.status, APRICT_STATUS_BAD_GEOMETRY);
+                if (needZ) {
+                    const double L = sqrt(ab_dot(Ps, Ps)), iL = 1.0 / L;
+                    cv.zl[0] = (float)(Ps.x * iL);
+                    cv.zl[1] = (float)(Ps.y * iL);
+                    cv.zl[2] = (float)((Ps.x * iL) * c0s.x + (Ps.y * iL) * c0s.y);
+                    cv.invL = (float)iL;
+                }
+                if (!RAYCAST) cv.kfast = (float)(P.vwd * P.vwd * P.vwd * Dn * Dn / (sqrt(uu) * sqrt(vv)));
+                cv.sxw = sp.source_pos.x;
+                cv.syw = sp.source_pos.y;
+            }
+            __syncthreads();
+            if (!col_live) continue;  // warp-uniform
+            // each view's products are added one view late: its gathers are in
+            // flight while the next view's rows are computed
+            f32x2 pvp[XB / 2];
+#pragma unroll
+            for (int k = 0; k < XB / 2; ++k) pvp[k] = pk(0.f, 0.f);
+            float wp = 0.f;
+            f32x2 acc2[XB / 2];
+#pragma unroll
+            for (int k = 0; k < XB / 2; ++k) acc2[k] = pk(0.f, 0.f);
+
+            for (int g0 = 0; g0 < cn; g0 += 32) {
+                __syncwarp();  // the previous group's records are no longer read
+                {
+                    const int t = g0 + lane;
+                    ColRec rec;
+                    rec.a = make_float4(0.f, 0.f, 0.f, 0.f);
+                    rec.b = make_uint4(0u, 0u, 0u, 0u);
+                    if (t < cn && sm.view[t].ok) {
+                        const ColView &cv = sm.view[t];
+                        const double D = fma(cv.d.den[0], X, fma(cv.d.den[1], Y, cv.d.den[3]));
+                        const double rD = 1.0 / D;
+                        const double fu = fma(cv.d.nu[0], X, fma(cv.d.nu[1], Y, cv.d.nu[3])) * rD;
+                        if (fabs(fu) < 4194304.0) {  // else (also D = 0) off the detector
+                            int iu = BILIN ? __double2int_rd(fu) : __double2int_rn(fu);
+                            const float du = (float)(fu - (double)iu);
+                            if (!BILIN && fabsf(du) > 0.499f)
+                                iu = refine_index(cv.d.nu, cv.d.den, VoxRef{X, Y, 0.0}, iu, du);
+                            if (BILIN ? fu > -1.0 && iu < (int)P.nu : (unsigned)iu < P.nu) {
+                                const double A = fma(cv.d.nv[0], X, fma(cv.d.nv[1], Y, fma(cv.d.nv[2], Z0, cv.d.nv[3]))) * rD -
+                                                 (double)crow;
+                                const double S = cv.d.nv[2] * P.vwd * rD;
+                                const float Af = (float)A, Sf = (float)S;
+                                const float frD = (float)rD;
+                                float w = RAYCAST ? 1.f : cv.kfast * (frD * frD);
+                                if (needZ) {
+                                    const float Z = fmaf(cv.zl[0], (float)X, fmaf(cv.zl[1], (float)Y, cv.zl[2]));
+                                    if (P.pL != 0) w *= powi_fast(Z * cv.invL, P.pL);
+                                    if (P.pV != 0) w *= powi_fast(Z * P.inv_val, P.pV);
+                                    if (RAYCAST && P.preset != 0)
+                                        w *= preset_weight(P.preset, P.val, (float)X + P.c0[0], (float)Y + P.c0[1], cv.sxw,
+                                                           cv.syw, Z);
+                                }
+                                const float cu = fabsf((float)(fu - 0.5 * ((double)P.nu - 1.0)));
+                                if (P.sep > 0.f) w *= ab_edge_taper_half(cu, 2.f / (float)P.nu, P.inv_sep);
+                                // error of the FP32 row coordinate, with a margin of 1.5, and where each
+                                // block of 32 voxels projects (with that error to spare)
+                                const float eps = fmaf(1.5f * 5.9604645e-8f,
+                                                       3.f * fabsf(Af) + (3.f * 32 * XB) * fabsf(Sf) + (float)P.nv, 1e-6f);
+                                unsigned in = 0, across = 0;
+#pragma unroll
+                                for (int k = 0; k < XB; ++k) {
+                                    const float e0 = fmaf((float)(32 * k), Sf, Af) - coff;
+                                    const float e1 = fmaf((float)(32 * k + 31), Sf, Af) - coff;
+                                    const float lo = fminf(e0, e1), hi = fmaxf(e0, e1);
+                                    if (lo - eps >= -insidev && hi + eps <= insidev)
+                                        in |= 1u << k;
+                                    else if (!(lo - eps > offv || hi + eps < -offv))
+                                        across |= 1u << k;
+                                }
+                                const uint64_t col = (uint64_t)(uintptr_t)(P.projs + (int64_t)(v0 + t) * P.stride_view +
+                                                                           (int64_t)iu * P.su + (int64_t)crow * P.sv) -
+                                                     4ull * 0x4B400000ull * (uint64_t)(uint32_t)P.sv;
+                                unsigned cols = 3u;  // which of the two columns lie on the detector
+                                if (BILIN && (iu < 0 || iu + 1 >= (int)P.nu)) {
+                                    cols = (iu >= 0 ? 1u : 0u) | (iu + 1 < (int)P.nu ? 2u : 0u);
+                                    across |= in;
+                                    in = 0u;
+                                }
+                                rec.a = make_float4(Af, Sf, w, BILIN ? du : 0.5f - eps);
+                                rec.b = make_uint4((uint32_t)col, (uint32_t)(col >> 32), (in & pairs) | (across & blocks) << 8,
+                                                   cols);
+                            }
+                        }
+                    }
+                    sm.rec[warp][lane] = rec;
+                }
+                __syncwarp();
+                const int gn = min(32, cn - g0);
+                for (int j = 0; j < gn; ++j) {
+                    const ColRec &rc = sm.rec[warp][j];
+                    const uint4 rb = rc.b;
+                    if (rb.z == 0u) continue;  // off the detector (warp-uniform)
+                    const float4 ra = rc.a;
+                    const uint64_t col = ((uint64_t)rb.y << 32) | rb.x;
+                    const float a = fmaf((float)lane, ra.y, ra.x), s32 = 32.f * ra.y;
+                    const f32x2 w2 = pk(wp, wp);
+                    wp = ra.z;
+                    const f32x2 f0 = pk(a, a + s32), s2 = pk(s32, s32);
+                    const unsigned in = rb.z & 255u, across = rb.z >> 8;
+                    float tie = 0.f;
+                    const uint64_t col1 = col + su4;                                  // BILIN: the second column,
+                    const f32x2 fx2 = pk(ra.w, ra.w), gx2 = pk(1.f - ra.w, 1.f - ra.w);  // the columns' weights
+                    const f32x2 wc2 = pk(ra.z, ra.z);
+                    // two blocks (voxels l + 64 k and l + 64 k + 32) inside the flat box
+                    auto inner_pair = [&](int k) {
+                        const f32x2 f = k == 0 ? f0 : fma2(pk(2.f * k, 2.f * k), s2, f0);
+                        if constexpr (BILIN) {
+                            const f32x2 t = add2(add2(f, mhalf), magic);  // floor(f) (or f - 1 for an integer f)
+                            const f32x2 fy = fma2(add2(t, nmagic), minus1, f);
+                            float ta, tb;
+                            upk(t, ta, tb);
+                            const char *pa = reinterpret_cast<const char *>(col + (uint64_t)(uint32_t)__float_as_int(ta) * sv4);
+                            const char *pb = reinterpret_cast<const char *>(col + (uint64_t)(uint32_t)__float_as_int(tb) * sv4);
+                            const char *qa = reinterpret_cast<const char *>(col1 + (uint64_t)(uint32_t)__float_as_int(ta) * sv4);
+                            const char *qb = reinterpret_cast<const char *>(col1 + (uint64_t)(uint32_t)__float_as_int(tb) * sv4);
+                            auto at = [](const char *p, int o) { return __ldg(reinterpret_cast<const float *>(p) + o); };
+                            const f32x2 v00 = pk(at(pa, 0), at(pb, 0)), v01 = pk(at(pa, 1), at(pb, 1));
+                            const f32x2 v10 = pk(at(qa, 0), at(qb, 0)), v11 = pk(at(qa, 1), at(qb, 1));
+                            const f32x2 t1 = fma2(v10, fx2, mul2(v00, gx2)), t2 = fma2(v11, fx2, mul2(v01, gx2));
+                            const f32x2 pv = fma2(t2, fy, mul2(t1, fma2(fy, minus1, one)));
+                            acc2[k] = fma2(pv, wc2, acc2[k]);
+                            return;
+                        }
+                        const f32x2 t = add2(f, magic);
+                        const f32x2 d = fma2(add2(t, nmagic), minus1, f);  // f - round(f)
+                        float ta, tb, da, db;
+                        upk(t, ta, tb);
+                        upk(d, da, db);
+                        tie = fmaxf(tie, fmaxf(fabsf(da), fabsf(db)));
+                        const float pa = __ldg(reinterpret_cast<const float *>(col + (uint64_t)(uint32_t)__float_as_int(ta) * sv4));
+                        const float pb = __ldg(reinterpret_cast<const float *>(col + (uint64_t)(uint32_t)__float_as_int(tb) * sv4));
+                        acc2[k] = fma2(pvp[k], w2, acc2[k]);
+                        pvp[k] = pk(pa, pb);
+                    };
+                    // one block across the flat box's or the detector's edge
+                    auto edge_block = [&](int k) -> float {
+                        // (a lane past the volume's top gathers along where its row exists; never written)
+                        if (!((in | across) >> k & 1u)) return 0.f;  // warp-uniform
+                        const float fo = (k & 1) ? a + s32 : a;
+                        const float f = fminf(fmaxf(k < 2 ? fo : fmaf((float)(k & ~1), s32, fo), -2097152.f), 2097152.f);
+                        if constexpr (BILIN) {
+                            const float fl = floorf(f), fy = f - fl;
+                            const int j0 = (int)fl + crow;
+                            const float *p = reinterpret_cast<const float *>(col + 4ull * 0x4B400000ull) + (j0 - crow);
+                            const bool r0 = (unsigned)j0 < P.nv, r1 = (unsigned)(j0 + 1) < P.nv, c0 = rb.w & 1u, c1 = rb.w & 2u;
+                            const float v00 = r0 && c0 ? __ldg(p) : 0.f, v01 = r1 && c0 ? __ldg(p + 1) : 0.f;
+                            const float v10 = r0 && c1 ? __ldg(p + P.su) : 0.f, v11 = r1 && c1 ? __ldg(p + P.su + 1) : 0.f;
+                            const float t1 = v00 * (1.f - ra.w) + v10 * ra.w, t2 = v01 * (1.f - ra.w) + v11 * ra.w;
+                            float pv = t1 * (1.f - fy) + t2 * fy;
+                            const float rv = fabsf(f - coff);
+                            if (P.sep > 0.f && rv > flatv && pv != 0.f) pv *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
+                            return pv;
+                        }
+                        const float t = __fadd_rn(f, kMagic);
+                        const int i = __float_as_int(t) - 0x4B400000 + crow;
+                        float pv = ldg_if(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4, (unsigned)i < P.nv);
+                        if (fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) > ra.w)
+                            pv = col_exact_row(sm.view[g0 + j].d, X, Y, fma((double)(lane + 32 * k), P.vwd, Z0), f, crow,
+                                               (int)P.nv, col, sv4);
+                        const float rv = fabsf(f - coff);
+                        if (P.sep > 0.f && rv > flatv && pv != 0.f) pv *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
+                        return pv;
+                    };
+                    if (in == kAll) {  // the whole column
+#pragma unroll
+                        for (int k = 0; k < XB / 2; ++k) inner_pair(k);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < XB / 2; ++k) {  // warp-uniform branches
+                            if ((in >> (2 * k) & 3u) == 3u) {
+                                inner_pair(k);
+                            } else {
+                                if (!BILIN) {
+                                    acc2[k] = fma2(pvp[k], w2, acc2[k]);
+                                    pvp[k] = pk(0.f, 0.f);
+                                }
+                                if ((in | across) >> (2 * k) & 3u) {
+                                    const f32x2 e = pk(edge_block(2 * k), edge_block(2 * k + 1));
+                                    if (BILIN)
+                                        acc2[k] = fma2(e, wc2, acc2[k]);
+                                    else
+                                        pvp[k] = e;
+                                }
+                            }
+                        }
+                    }
+                    if (!BILIN && tie > ra.w) {  // some row of this lane is too close to call in FP32
+#pragma unroll
+                        for (int k = 0; k < XB; ++k) {
+                            const float fo = (k & 1) ? a + s32 : a;
+                            const float f = k < 2 ? fo : fmaf((float)(k & ~1), s32, fo);
+                            const float d = __fsub_rn(f, __fsub_rn(__fadd_rn(f, kMagic), kMagic));
+                            if (!(in >> k & 1u) || fabsf(d) <= ra.w) continue;
+                            const float pe = col_exact_row(sm.view[g0 + j].d, X, Y, fma((double)(lane + 32 * k), P.vwd, Z0), f,
+                                                           crow, (int)P.nv, col, sv4);
+                            float q0, q1;
+                            upk(pvp[k / 2], q0, q1);
+                            pvp[k / 2] = (k & 1) ? pk(q0, pe) : pk(pe, q1);
+                        }
+                    }
+                }
+            }
+            // the chunk's partial sums into the compensated totals
+            const f32x2 w2 = pk(wp, wp);
+            float acc[XB];
+#pragma unroll
+            for (int k = 0; k < XB / 2; ++k) upk(fma2(pvp[k], w2, acc2[k]), acc[2 * k], acc[2 * k + 1]);
+#pragma unroll
+            for (int k = 0; k < XB; ++k) {
+                const int i = lane + 32 * k;
+                const float sk = ksum[i];
+                const float y = acc[k] - kcomp[i];
+                const float tk = sk + y;
+                kcomp[i] = (tk - sk) - y;
+                ksum[i] = tk;
+            }
+        }
+    }
+    if (col_live) {
+#pragma unroll
+        for (int k = 0; k < XB; ++k) {
+            const int i = lane + 32 * k;
+            const float total = ksum[i] - kcomp[i];
+            const float value = n_sub == 1 ? total : total / (float)n_sub;
+            if (z0 + i >= P.n[2] || value == 0.f) continue;  // the reference skips the write (:1010)
+            const int64_t o = (int64_t)ix * P.vs[0] + (int64_t)iy * P.vs[1] + (int64_t)(z0 + i) * P.vs[2];
+            const float m = P.mult ? __ldcs(P.mult + o) : 1.f;
+            __stcs(P.vol + o, value * m + __ldcs(P.vol + o));
+        }
+    }
+}
+
+}  // namespace ab_bp

@@ -187,6 +187,27 @@ APRICT_API int aprict_b200_backproject(const aprict_proj_spec *specs_dev,
                             uint32_t *status_dev, aprict_stream_t stream);
 
 
+/* The same with what the caller knows of the views. A view is upright when
+ * its det_u has no z component and its det_v no x and y components (and, with
+ * Z factors or a weighting preset, source and detector centre lie at one
+ * height); calls whose views are all upright have a faster kernel. Without a
+ * promise both kernels are launched and each looks at the views itself.
+ *   views: APRICT_VIEWS_UNKNOWN, APRICT_VIEWS_UPRIGHT (a promise: the result is
+ *          undefined if a view is not upright) or APRICT_VIEWS_GENERAL (the
+ *          general kernel whatever the views)                              */
+#define APRICT_VIEWS_UNKNOWN 0u
+#define APRICT_VIEWS_UPRIGHT 1u
+#define APRICT_VIEWS_GENERAL 2u
+APRICT_API int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev,
+                                  const aprict_proj_desc *projs,
+                                  const float *projs_dev,
+                                  const aprict_vol_desc *vol, float *vol_dev,
+                                  const float *multiplier_dev,
+                                  const aprict_backproject_config *cfg,
+                                  uint32_t views, uint32_t *status_dev,
+                                  aprict_stream_t stream);
+
+
 /* ---- Element-wise volume operations (linear float32 buffers of n elements).
  * Replace the surface kernels of texture_operations.cu driven by
  * src/aprict/lib/texture_tools/operations.py. ---- */
@@ -455,6 +476,12 @@ APRICT_API size_t aprict_b200_batch_plan_bytes(int op, int n_scans);
  * bilinear) in every scan. The plan records the device pointers given here. */
 APRICT_API int aprict_b200_batch_plan(int op, const aprict_scan *scans, int n_scans, const void *configs,
                                       void *plan_host, size_t plan_capacity);
+
+/* The same with what the caller knows of each scan's views (APRICT_VIEWS_*, one
+ * per scan, as in aprict_b200_backproject_views; NULL: nothing). Only
+ * backprojection plans use it. */
+APRICT_API int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, int n_scans, const void *configs,
+                                            const uint32_t *views, void *plan_host, size_t plan_capacity);
 
 /* Run a plan: plan_dev is a byte copy of plan_host in device memory (256-byte
  * aligned). The work counters in plan_dev must be zero before the first run

@@ -1,0 +1,144 @@
+"""The z-column backprojection of upright views (ab_bpcol.cuh) at the edges of its blocks.
+
+A warp takes a column of 32 XB voxels in blocks of 32, in pairs; a block lies
+inside the detector's flat box, across its edge or off the detector; calls
+with a view that is not upright take the brick kernel. Against the FP64 oracle:
+rel L2 <= 1e-5, the gate of every backprojection mode. Against the brick kernel
+(``APRICT_VIEWS_GENERAL``) on the same call: both settle the nearest rows in
+FP64 and sum in FP32 (<= 1e-6); bilinear coordinates carry the brick kernel's FP32
+error of about 1e-4 pixel (<= 1e-5).
+"""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from aprict_b200 import Volume, geometry
+from aprict_b200.batch import ScanBatch
+from aprict_b200.cb import flatpanel as fp
+from helpers import circular, jittered, rel_l2
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+MODES = {
+    "nearest": dict(fast_approx=True),
+    "nearest-taper": dict(fast_approx=True, cyl_mask_rad=7.0, soften_det_edges_proportion=0.2),
+    "bilinear": dict(fast_approx=True, approx_mode_bilinear_interpolate=True),
+    "bilinear-taper": dict(fast_approx=True, approx_mode_bilinear_interpolate=True, soften_det_edges_proportion=0.2),
+    "raycast": dict(fast_approx=True, approx_mode_direct_raycast=True, Z_on_val_factor_power=-2, Z_on_val_factor_val=100.0),
+    "raycast-preset": dict(fast_approx=True, approx_mode_direct_raycast=True, Z_on_val_factor_power=-1,
+                           Z_on_val_factor_val=100.0, backproj_weighting_preset=1),
+    "raycast-bilinear": dict(fast_approx=True, approx_mode_direct_raycast=True, approx_mode_bilinear_interpolate=True,
+                             Z_on_L_factor_power=-1),
+    "sub-samples": dict(fast_approx=True, ssx=1, ssy=2, ssz=2),
+}
+
+
+def _run(mode: str, pg: fp.ProjGeom, data: torch.Tensor, shape, order="C", views: int | None = None, vw: float = 1.0) -> np.ndarray:
+    v = Volume.zeros(shape, voxwid=vw, order=order)
+    ps = fp.ProjectionSet(pg, data=data)
+    if views is not None:
+        ps._backproject_promise = lambda needs_z: views  # noqa: SLF001
+    fp.backproject(fp.ConfigBackproject(**MODES[mode]), v, ps, block=True)
+    return v.as_numpy()
+
+
+def _data(pg: fp.ProjGeom, seed: int = 0) -> torch.Tensor:
+    a = np.random.default_rng(seed).random((pg.num_projs, int(pg.nu.flat[0]), int(pg.nv.flat[0]))).astype(np.float32)
+    return torch.from_numpy(a).cuda()
+
+
+def _oracle(mode: str, pg: fp.ProjGeom, data: torch.Tensor, shape, vw: float = 1.0) -> np.ndarray:
+    return O.backproject(pg.to_proj_spec_array(), data.cpu().numpy(), shape, fp.ConfigBackproject(**MODES[mode]).contents,
+                         voxwid=vw, corner=-np.float32(vw) * np.array(shape, np.float32) / 2)
+
+
+@pytest.mark.parametrize("nz", [2, 31, 32, 33, 64, 65, 128, 129, 160, 257])
+@pytest.mark.parametrize("mode", ["nearest-taper", "bilinear", "raycast"])
+def test_heights_match_oracle(nz: int, mode: str) -> None:
+    """Heights around the 32-voxel blocks, their pairs and the 2 / 4 / 8 voxels per thread; the detector
+    cuts the tall ones off at the top and bottom."""
+    shape = (9, 17, nz)
+    pg = circular(70, 160, 120, 0.913, 25, 63)  # more than one chunk of 64 views
+    data = _data(pg, nz)
+    want = _oracle(mode, pg, data, shape)
+    assert np.linalg.norm(want) > 0
+    got = _run(mode, pg, data, shape)
+    assert rel_l2(got, want) <= 1e-5
+    assert rel_l2(_run(mode, pg, data, shape, views=0), got) == 0  # no promise: the same kernel after its own look
+    assert rel_l2(_run(mode, pg, data, shape, views=2), got) <= (1e-5 if "bilinear" in mode else 1e-6)
+
+
+@pytest.mark.parametrize("order", ["C", "F"])
+@pytest.mark.parametrize("mode", sorted(MODES))
+def test_modes_match_oracle(mode: str, order: str) -> None:
+    shape = (20, 13, 70)
+    pg = geometry.helical_scan(n_views=40, R=90.0, L_minus_R=70.0, pix_at_iso=0.637, nu=41, nv=38, pitch=1.2, theta_start=0.31)
+    data = _data(pg, 5)
+    want = _oracle(mode, pg, data, shape)
+    assert np.linalg.norm(want) > 0
+    assert rel_l2(_run(mode, pg, data, shape, order), want) <= 1e-5
+
+
+@pytest.mark.parametrize("layout", ["v strided", "u fastest", "views strided"])
+@pytest.mark.parametrize("mode", ["nearest", "bilinear", "raycast"])
+def test_projection_strides(mode: str, layout: str) -> None:
+    """The column address is formed from the strides; bilinear with v not contiguous takes the bricks."""
+    shape = (12, 10, 40)
+    pg = circular(12, 120, 100, 0.713, 26, 44)
+    data = _data(pg, 3)
+    if layout == "v strided":
+        view = torch.empty((12, 26, 44, 3), device="cuda")[..., 1].copy_(data)
+    elif layout == "u fastest":
+        view = torch.empty((12, 44, 26), device="cuda").transpose(1, 2).copy_(data)
+    else:
+        view = torch.empty((12, 2, 26, 44), device="cuda")[:, 1].copy_(data)
+    assert rel_l2(_run(mode, pg, view, shape), _run(mode, pg, data, shape)) <= (1e-5 if mode == "bilinear" else 1e-6)
+
+
+@pytest.mark.parametrize("mode", ["nearest", "bilinear", "raycast"])
+def test_tilted_and_mixed_views_take_the_bricks(mode: str) -> None:
+    shape = (14, 12, 50)
+    pg = circular(20, 120, 100, 0.713, 40, 44)
+    tilted = jittered(np.random.default_rng(2), pg)
+    vecs = {k: np.broadcast_to(getattr(pg, k), (20, 3)).copy() for k in ("source_pos", "det_pos", "det_uvec", "det_vvec")}
+    for k in vecs:
+        vecs[k][7] = getattr(tilted, k)[7]  # one view of twenty
+    mixed = fp.ProjGeom(**vecs, nu=pg.nu, nv=pg.nv)
+    for g in (tilted, mixed):
+        data = _data(g, 4)
+        want = _oracle(mode, g, data, shape)
+        assert rel_l2(_run(mode, g, data, shape), want) <= 1e-5
+        assert rel_l2(_run(mode, g, data, shape, views=0), want) <= 1e-5
+
+
+def test_non_finite_pixels_stay_where_they_project() -> None:
+    """An infinite and a NaN pixel reach the voxels that take them and no others."""
+    shape = (16, 16, 96)
+    pg = circular(6, 200, 150, 0.8137, 40, 140)
+    data = _data(pg, 6)
+    clean = _run("nearest", pg, data, shape)
+    data[2, 20, 70], data[4, 11, 33] = float("inf"), float("nan")
+    got, bricks = _run("nearest", pg, data, shape), _run("nearest", pg, data, shape, views=2)
+    assert not np.isfinite(got).all()
+    np.testing.assert_array_equal(np.isfinite(got), np.isfinite(bricks))
+    ok = np.isfinite(got)
+    assert rel_l2(got[ok], clean[ok]) <= 1e-6
+
+
+@pytest.mark.parametrize("mode", ["nearest", "bilinear", "raycast"])
+def test_batch_of_upright_and_tilted_scans(mode: str) -> None:
+    """A batch runs the columns of its upright scans and the bricks of the others; each equals its one-scan call."""
+    rng = np.random.default_rng(8)
+    shapes = [(20, 18, 24), (10, 30, 150), (33, 9, 70), (12, 12, 40)]
+    pgs = [circular(15, 120, 100, 0.713, 50, 52), circular(9, 140, 90, 0.61, 40, 60, theta0=0.4),
+           jittered(rng, circular(12, 120, 100, 0.713, 50, 52)), jittered(rng, circular(20, 130, 100, 0.66, 44, 40))]
+    cfg = fp.ConfigBackproject(**MODES[mode])
+    datas = [_data(g, i) for i, g in enumerate(pgs)]
+    vols = [Volume.zeros(s, voxwid=1.0) for s in shapes]
+    ScanBatch(vols, [fp.ProjectionSet(g, data=d) for g, d in zip(pgs, datas)]).backproject(cfg, block=True)
+    for s, g, d, v in zip(shapes, pgs, datas, vols):
+        assert rel_l2(v.as_numpy(), _run(mode, g, d, s)) <= 1e-6
