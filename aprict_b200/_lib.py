@@ -37,6 +37,9 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
         _c_int,
         [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     ),
+    "aprict_b200_backproject_slices": (
+        _c_int, [_c_void_p, ctypes.c_uint32, ctypes.c_uint32, _c_void_p, ctypes.c_int64, ctypes.c_int32] + [_c_void_p] * 5,
+    ),
     "aprict_b200_backproject_views": (
         _c_int, [_c_void_p] * 7 + [ctypes.c_uint32, _c_void_p, _c_void_p],
     ),

@@ -113,11 +113,34 @@ class RampFilterer:
             raise ValueError(msg)
         if outs is None:
             outs = [torch.empty_like(data) for _ in self._taps]
+        if weights is not None and (tuple(weights.shape) != tuple(data.shape[1:]) or weights.dtype != torch.float32):
+            msg = "weights must be a float32 (nu, nv) tensor"
+            raise ValueError(msg)
+        return self._filter_rows(data, weights, scale, outs)
+
+    def filter_interleaved(self, data: torch.Tensor, n_slices: int, *, weights: torch.Tensor, scale: float = 1.0) -> torch.Tensor:
+        """Filter the ``n_slices`` sinograms stacked in (n_slices * M, nu, 1) data into one
+        (M * nu + 1, pitch) tensor with the slices interleaved (slice s of view m, sample u at
+        [m * nu + u, s]; pitch a multiple of 4, the rest of a row undefined) and a last row of
+        zeros: the layout of ``aprict_b200_backproject_slices``. One filter, (nu, 1) weights."""
+        nu = self.chunk_shape[1]
+        if data.dim() != 3 or tuple(data.shape[1:]) != (nu, 1) or data.shape[0] % n_slices or self.num_kerns != 1:
+            msg = "Input projection array shape does not match the shape initialised for this filtering object."
+            raise ValueError(msg)
+        if data.dtype != torch.float32 or not data.is_cuda:
+            msg = "data must be a float32 CUDA tensor"
+            raise ValueError(msg)
+        m = data.shape[0] // n_slices
+        pitch = (n_slices + 3) // 4 * 4
+        out = torch.empty((m * nu + 1, pitch), dtype=torch.float32, device=data.device)
+        out[-1].zero_()
+        src = data.unflatten(0, (n_slices, m))[..., 0].permute(1, 2, 0)  # (m, nu, slice)
+        self._filter_rows(src, weights.expand(nu, n_slices), scale, [out[:-1].view(m, nu, pitch)[..., :n_slices]])
+        return out
+
+    def _filter_rows(self, data: torch.Tensor, weights: torch.Tensor | None, scale: float, outs: list[torch.Tensor]) -> list[torch.Tensor]:
         wptr, wsu, wsv = None, 0, 0
         if weights is not None:
-            if tuple(weights.shape) != tuple(data.shape[1:]) or weights.dtype != torch.float32:
-                msg = "weights must be a float32 (nu, nv) tensor"
-                raise ValueError(msg)
             wptr, (wsu, wsv) = weights.data_ptr(), weights.stride()
         din = _desc(data)
         lib = _lib.lib()

@@ -39,6 +39,7 @@ import torch
 
 import math
 
+from . import _lib
 from .cb import flatpanel as fp
 from .cb.ramp_filter import FBPFilterer
 from .volume import Volume
@@ -103,6 +104,43 @@ def fbp_fan_circ(
     return volume
 
 
+_SLICES_PER_CALL = 64  # slices per aprict_b200_backproject_slices call
+_MIN_STACK = 4  # fewer slices are backprojected one by one
+
+
+def _one_scan_stack(projs: list[fp.ProjectionSet], volumes: list[Volume]) -> bool:
+    """Whether the slices share one scan and one grid whose plane holds every source and
+    detector row, so that they can be backprojected together (``aprict_b200_backproject_slices``)."""
+    if len(projs) < _MIN_STACK:
+        return False
+    sp, v0 = projs[0].proj_specs, volumes[0]
+    z = float(v0.corner[2]) + 0.5 * float(np.float32(v0.voxwid))  # the plane of the slices
+    if not (sp.ndim == 1 and np.all(sp["nv"] == 1) and np.all(sp["det_u"]["z"] == 0) and np.all(sp["det_v"]["x"] == 0)
+            and np.all(sp["det_v"]["y"] == 0) and np.all(sp["source_pos"]["z"] == z) and np.all(sp["det_pos"]["z"] == z)):
+        return False
+    if any(p.proj_geom is not projs[0].proj_geom and not np.array_equal(p.proj_specs, sp) for p in projs):
+        return False
+    pos = v0.pos_c
+    return v0.shape[2] == 1 and all(
+        v.shape == v0.shape and v.order == "C" and v.voxwid == v0.voxwid and v.data.is_cuda and v.data.dtype == torch.float32
+        and np.array_equal(v.pos_c, pos) for v in volumes
+    )
+
+
+def _backproject_slices(cfg: fp.ConfigBackproject, projs: fp.ProjectionSet, data: torch.Tensor, volumes: list[Volume],
+                        nu: int) -> None:
+    """Add the backprojection of interleaved slices (``RampFilterer.filter_interleaved``) into ``volumes``."""
+    ptrs = np.array([v.data.data_ptr() for v in volumes], dtype=np.uint64)
+    conf, vd = cfg.contents, volumes[0]._desc()  # noqa: SLF001
+    _lib.check(
+        _lib.lib().aprict_b200_backproject_slices(
+            projs.specs_device().data_ptr(), projs.proj_geom.num_projs, nu, data.data_ptr(), data.stride(0), len(volumes),
+            _lib.ptr(vd), _lib.ptr(ptrs), _lib.ptr(conf), None, torch.cuda.current_stream().cuda_stream,
+        ),
+        "backproject_slices",
+    )
+
+
 def fbp_fan_circ_batch(
     projs: list[fp.ProjectionSet],
     volumes: list[Volume],
@@ -140,12 +178,19 @@ def fbp_fan_circ_batch(
     if stacked is None:
         stacked = torch.cat([p.data.float() for p in projs], dim=0)
     filt = FBPFilterer(L=L, physpixwid=pixwid, proj_2d_shape=(nu, nv), _hacky_fan_beam_mode=True, apodization=apodization)
-    (filtered,) = filt.rfilt.filter(stacked, weights=filt._weights, scale=1.0 / (4.0 * np.pi * R * m))  # noqa: SLF001
+    scale = 1.0 / (4.0 * np.pi * R * m)
     support = R * np.sin(np.arctan(pixwid * nu / 2 / L))
     cfg = fp.ConfigBackproject(
         fast_approx=True, cyl_mask_rad=support, Z_on_val_factor_power=-2, Z_on_val_factor_val=R,
         approx_mode_direct_raycast=True, approx_mode_bilinear_interpolate=interpolate,
     )
+    if not interpolate and stacked.shape[0] == len(projs) * m and _one_scan_stack(projs, volumes):
+        for a in range(0, len(projs), _SLICES_PER_CALL):
+            n = min(_SLICES_PER_CALL, len(projs) - a)
+            data = filt.rfilt.filter_interleaved(stacked[a * m : (a + n) * m], n, weights=filt._weights, scale=scale)  # noqa: SLF001
+            _backproject_slices(cfg, projs[0], data, volumes[a : a + n], nu)
+        return volumes
+    (filtered,) = filt.rfilt.filter(stacked, weights=filt._weights, scale=scale)  # noqa: SLF001
     views = [p._with_data(filtered[i * m : (i + 1) * m]) for i, p in enumerate(projs)]  # noqa: SLF001
     ScanBatch(volumes, views).backproject(cfg)
     return volumes

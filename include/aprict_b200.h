@@ -208,6 +208,22 @@ APRICT_API int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev,
                                   aprict_stream_t stream);
 
 
+/* Fan-beam backprojection of up to 64 slices that share one scan (detector of
+ * one row, every slice in the plane of its source and row centre): the
+ * nearest-pixel direct-raycast mode of aprict_b200_backproject, every slice's
+ * image in one launch.
+ *   data_dev: the slices' filtered data interleaved, (n_views, nu, pitch) floats,
+ *             slices 0 .. n_slices - 1 first in each pixel, then one more pixel
+ *             of zeros; 16-byte aligned, pitch a multiple of 4 up to 64
+ *   vol     : the slices' common grid (nz = 1, C order)
+ *   vols_dev: n_slices device pointers (a host array): vols[s] += BP(slice s) */
+APRICT_API int aprict_b200_backproject_slices(const aprict_proj_spec *specs_dev, uint32_t n_views,
+                                   uint32_t nu, const float *data_dev, int64_t pitch,
+                                   int32_t n_slices, const aprict_vol_desc *vol,
+                                   float *const *vols_dev, const aprict_backproject_config *cfg,
+                                   uint32_t *status_dev, aprict_stream_t stream);
+
+
 /* ---- Element-wise volume operations (linear float32 buffers of n elements).
  * Replace the surface kernels of texture_operations.cu driven by
  * src/aprict/lib/texture_tools/operations.py. ---- */

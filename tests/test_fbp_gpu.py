@@ -90,3 +90,54 @@ def test_batched_slices_equal_single_slice_fbp() -> None:
     for o, w in zip(outs, singles):
         assert np.linalg.norm(w) > 0
         assert rel_l2(o.as_numpy(), w) <= 1e-6
+
+
+@pytest.mark.parametrize(("slices", "n", "nu"), [(4, 40, 90), (5, 33, 128), (9, 50, 200), (17, 21, 96), (33, 70, 150),
+                                                 (64, 24, 140), (67, 20, 130)])
+def test_slice_stack_equals_single_slices(slices: int, n: int, nu: int) -> None:
+    """Stacks of one scan run through the interleaved kernel: slice counts around its lane groups (4 slices
+    a lane, 1 to 16 lanes) and past one call's 64, slices narrower than a tile, rows filtered directly
+    (nu < 128) and by FFT. Each slice equals its own reconstruction up to FP32 rounding."""
+    from aprict_b200.recon import fbp_fan_circ_batch
+
+    pg = circular(75, 120.0, 100.0, 0.9 * n * 0.5 / nu * 1.2345, nu, 1, theta0=0.21)
+    rng = np.random.default_rng(slices)
+    projs, vols, want = [], [], []
+    for _ in range(slices):
+        ps = fp.ProjectionSet(pg, data=rng.random((75, nu, 1)).astype(np.float32))
+        one = Volume.zeros((n, n + 3, 1), voxwid=0.5)
+        fbp_fan_circ(ps, one)
+        projs.append(ps)
+        want.append(one.as_numpy())
+        vols.append(Volume.zeros((n, n + 3, 1), voxwid=0.5))
+        vols[-1].fill(0.25)  # added to
+    fbp_fan_circ_batch(projs, vols)
+    for v, w in zip(vols, want):
+        assert np.linalg.norm(w) > 0
+        assert rel_l2(v.as_numpy() - 0.25, w) <= 2e-6
+
+
+@pytest.mark.parametrize("case", ["off plane", "other views", "F order", "other grid", "bilinear"])
+def test_slice_stacks_that_do_not_share_a_scan_go_one_by_one(case: str) -> None:
+    from aprict_b200.recon import fbp_fan_circ_batch
+
+    n, nu = 40, 130
+    pgs = [circular(60, 120.0, 100.0, 0.21, nu, 1, theta0=0.21) for _ in range(5)]
+    order, shapes, z = "C", [(n, n, 1)] * 5, 0.0
+    if case == "other views":
+        pgs[3] = circular(60, 120.0, 100.0, 0.21, nu, 1, theta0=0.9)
+    elif case == "F order":
+        order = "F"
+    elif case == "other grid":
+        shapes = [(n, n, 1), (n, n + 8, 1)] + [(n, n, 1)] * 3
+    elif case == "off plane":
+        z = 0.05
+    rng = np.random.default_rng(3)
+    projs = [fp.ProjectionSet(g, data=rng.random((60, nu, 1)).astype(np.float32)) for g in pgs]
+    vols = [Volume.zeros(s, voxwid=0.5, order=order, pos_c=(0, 0, z)) for s in shapes]
+    fbp_fan_circ_batch(projs, vols, interpolate=case == "bilinear")
+    for p, s, v in zip(projs, shapes, vols):
+        one = Volume.zeros(s, voxwid=0.5, order=order, pos_c=(0, 0, z))
+        fbp_fan_circ(p, one, interpolate=case == "bilinear")
+        # (bilinear coordinates are stepped in FP32 from the thread's first voxel, two voxels against four)
+        assert rel_l2(v.as_numpy(), one.as_numpy()) <= (2e-5 if case == "bilinear" else 2e-6)
