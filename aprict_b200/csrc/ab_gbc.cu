@@ -434,12 +434,28 @@ __global__ void __launch_bounds__(kGThreads, BILIN ? 3 : 4) k_backproject_gbc_z(
 //   w(r, t, z) = A(r, t) cos^3(theta) s_v(sin^2 theta),
 //   A = c / max(1e-9, c^2 + (c - ell)^2) s_h(1 - c^2),
 //   cos theta = ell / h, sin^2 theta = z^2 / h^2, h^2 = ell^2 + z^2.
-// One thread per (radius, angle) evaluates A once and runs the height loop
-// (a reciprocal square root and a few multiplies per sample). sin^2 theta
-// grows with z, so the loop stops at the first height past the vertical
-// window, where the window is 0 (it reaches 0 continuously at its edge).
-// Heights are summed in FP32 in runs of 64, the runs in FP64; per radius an
-// FP64 block sum over angles and one atomic add.
+// The inner sum over heights is a function F of ell alone, smooth on the scale
+// of ell, so it is evaluated at kNodes values of ell over the call's range
+// (k_gbc_height_table, one warp each, the samples and weights of the rule) and
+// taken by four-point Lagrange interpolation for each (radius, angle): 4096
+// height sums instead of n_r num_ang of them (396 x 6000: 2.4 million).
+// Interpolation error, relative to F, node spacing h: (h / ell)^4 from the
+// smooth part, below 4e-9 where ell >= 128 h; and from the window, whose
+// second derivative jumps at its two edges by up to 6 gamma^2 (ds/d ell)^2,
+// |ds/d ell| <= 0.4 / ell: at a given ell only the samples within one node of
+// an edge feel it, a share of about h, hence at most 0.12 gamma^2 h^3 / ell^2,
+// 2e-8 for gamma <= 200 at h = 1.5e-4. Both lie below the FP32 rounding of the
+// samples. (radius, angle) pairs with ell < 128 h, and calls with a steeper
+// window (kMaxGamma) or without scratch for the table sum their heights directly.
+// 396 radii x 6000 x 6000 samples, the whole call: 7.0 -> 0.55 ms (most of it host
+// work; sums equal to 1e-8).
+// sin^2 theta grows with z, so a height sum stops at the first height past the
+// vertical window, where the window is 0 (it reaches 0 continuously at its
+// edge). Heights are summed in FP32 in runs of 64, the runs in FP64; per
+// radius an FP64 block sum over angles and one atomic add.
+constexpr int kNodes = 4096;        // interpolation nodes of the height sum
+constexpr int kDirectBelow = 128;   // node spacings below which ell is summed directly
+constexpr float kMaxGamma = 200.f;  // steepest window (1 / sine width of its band) that is interpolated
 constexpr int kZRun = 64;  // heights per FP32 partial sum
 
 // sum over heights iz = 0 .. num_z - 1 (iz = 0 with weight 1/2) of
@@ -490,20 +506,81 @@ __device__ double height_sum(float ell, int num_z, float dz, const SoftWin &v) {
     return tot;
 }
 
+// One lane's share of height_sum (heights 1 + lane, 33 + lane, ...): the same
+// samples and weights, a warp per ell.
+__device__ double height_sum_lane(float ell, int num_z, float dz, const SoftWin &v, int lane) {
+    const float e2 = ell * ell, e3 = e2 * ell;
+    double tot = lane == 0 ? 0.5 * (double)soft_of_sin2(0.f, v) : 0.0;
+    if (e3 == 0.f) return tot;
+    for (int iz = 1 + lane; iz < num_z;) {
+        float part = 0.f;
+        bool done = false;
+        for (int k = 0; k < kZRun && iz < num_z; ++k, iz += 32) {
+            const float z = (float)iz * dz;
+            const float ih = rsqrtf(fmaf(z, z, e2));
+            const float s = fabsf(z) * ih;
+            const float s2 = s * s;
+            if (s2 > v.sa2) {
+                done = true;
+                break;
+            }
+            const float win = s2 < v.sab2 ? 1.f : soft_cubic(s, v);
+            part = fmaf(e3 * ih * (ih * ih), win, part);
+        }
+        tot += (double)part;
+        if (done) break;
+    }
+    return tot;
+}
+
+// The nodes' range of ell: [|1 - r|, 1 + r] over the call's radii (increasing).
+__device__ __forceinline__ void ell_nodes(float r_max, float &lo, float &h) {
+    lo = fmaxf(0.f, 1.f - r_max);
+    h = (1.f + r_max - lo) / (float)(kNodes - 3);  // one node to spare at each end
+    lo -= h;
+}
+
+__global__ void __launch_bounds__(kGThreads) k_gbc_height_table(const float *r_on_R, int nr, double *table, int num_z, SoftWin v,
+                                                                float tan_v) {
+    const int lane = threadIdx.x & 31, node = (blockIdx.x * kGThreads + threadIdx.x) >> 5;
+    if (node >= kNodes) return;
+    float lo, h;
+    ell_nodes(r_on_R[nr - 1], lo, h);
+    const float dz = tan_v * (1.f + r_on_R[nr - 1]) / (float)(num_z - 1);
+    double s = height_sum_lane(fmaxf(0.f, fmaf((float)node, h, lo)), num_z, dz, v, lane);
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (lane == 0) table[node] = s;
+}
+
+// Four-point Lagrange interpolation of the height sum at ell.
+__device__ __forceinline__ double height_at(float ell, float lo, float h, const double *__restrict__ table) {
+    const double x = ((double)ell - (double)lo) / (double)h;
+    int i = (int)x;
+    i = i < 1 ? 1 : (i > kNodes - 3 ? kNodes - 3 : i);
+    const double t = x - (double)i;
+    const double a = __ldg(table + i - 1), b = __ldg(table + i), c = __ldg(table + i + 1), d = __ldg(table + i + 2);
+    const double t1 = t + 1.0, tm = t - 1.0, t2 = t - 2.0;
+    return (t1 * t * tm * d - t * tm * t2 * a) * (1.0 / 6.0) + (t1 * tm * t2 * b - t1 * t * t2 * c) * 0.5;
+}
+
+// table: the nodes' height sums, or null (every height sum taken directly).
 __global__ void __launch_bounds__(kGThreads) k_gbc_weight_integ(const float *r_on_R, int nr, double *out, int num_z,
-                                                                int num_ang, GbcSoft S, float tan_v) {
+                                                                int num_ang, GbcSoft S, float tan_v,
+                                                                const double *__restrict__ table) {
     __shared__ double warp_sums[kGThreads / 32];
     const float maxz = tan_v * (1.f + r_on_R[nr - 1]);  // tan(soft_vartheta_v) (1 + r_max)
     const float dz = maxz / (float)(num_z - 1);
-    const int ia = blockIdx.x * kGThreads + threadIdx.x;
-    const bool live = ia < num_ang;
-    const float t = (float)(live ? ia : 0) / (float)num_ang * 3.1415926535898f;
-    const float ct = cosf(t), st = sinf(t);
+    float lo, h;
+    ell_nodes(r_on_R[nr - 1], lo, h);
+    const float direct = table && h > 0.f ? fmaxf((float)kDirectBelow * h, lo + h) : INFINITY;
     const double mult = (double)((4.f * maxz * 3.1415926535898f) / ((float)num_z * (float)num_ang));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int r = blockIdx.y; r < nr; r += gridDim.y) {
         double w = 0.0;
-        if (live) {
+        for (int ia = blockIdx.x * kGThreads + threadIdx.x; ia < num_ang; ia += gridDim.x * kGThreads) {
+            const float t = (float)ia / (float)num_ang * 3.1415926535898f;
+            const float ct = cosf(t), st = sinf(t);
             const float rx = r_on_R[r] - ct, ry = -st;  // voxel minus source, in units of R
             const float q = rx * rx + ry * ry;
             const float rq = rsqrtf(q);
@@ -511,7 +588,10 @@ __global__ void __launch_bounds__(kGThreads) k_gbc_weight_integ(const float *r_o
             const float c = fmaxf(0.f, fminf(1.f, fabsf((rx * ct + ry * st) * rq)));  // NaN at q = 0 -> 1
             const float d = c - ell;
             const float a = __fdividef(c, fmaxf(1e-9f, c * c + d * d)) * soft_of_sin2(fmaxf(0.f, 1.f - c * c), S.h);
-            if (a != 0.f) w = (double)a * height_sum(ell, num_z, dz, S.v);
+            // (radii out of order may lie outside the nodes)
+            if (a != 0.f)
+                w += (double)a * (ell >= direct && ell <= fmaf((float)(kNodes - 2), h, lo) ? height_at(ell, lo, h, table)
+                                                                                          : height_sum(ell, num_z, dz, S.v));
         }
 #pragma unroll
         for (int k = 16; k > 0; k >>= 1) w += __shfl_xor_sync(0xffffffffu, w, k);
@@ -696,9 +776,15 @@ extern "C" int aprict_b200_backproject_gbc(const aprict_proj_spec *specs_dev, co
     return ab_cuda_check(cudaGetLastError(), "backproject_gbc launch");
 }
 
-extern "C" int aprict_b200_gbc_weight_integral(const float *r_on_R_dev, int32_t n_r, double *out_dev, int32_t num_z,
-                                               int32_t num_ang, const aprict_backproject_config *cfg,
-                                               aprict_stream_t stream) {
+extern "C" int64_t aprict_b200_gbc_weight_integral_scratch_bytes(int32_t n_r, int32_t num_ang) {
+    // The table pays from a few tables' worth of height sums on: 16384 of them in
+    // warps of 32 cost about what the table's 4096 warps do.
+    return (int64_t)n_r * num_ang >= 4 * (int64_t)kNodes ? (int64_t)(kNodes * sizeof(double)) : 0;
+}
+
+extern "C" int aprict_b200_gbc_weight_integral_scratch(const float *r_on_R_dev, int32_t n_r, double *out_dev, int32_t num_z,
+                                                       int32_t num_ang, const aprict_backproject_config *cfg,
+                                                       void *scratch_dev, aprict_stream_t stream) {
     if (cfg == nullptr) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "null backproject config");
     if (n_r <= 0) return APRICT_OK;
     if (r_on_R_dev == nullptr || out_dev == nullptr)
@@ -708,10 +794,29 @@ extern "C" int aprict_b200_gbc_weight_integral(const float *r_on_R_dev, int32_t 
     if (!finite_soft(cfg)) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "non-finite soft windows");
     const GbcSoft S{soft_win(cfg->soft_vartheta_v, cfg->soft_vartheta_v_softspan),
                     soft_win(cfg->soft_vartheta_h, cfg->soft_vartheta_h_softspan)};
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    const float tan_v = (float)tan((double)cfg->soft_vartheta_v);
+    if ((reinterpret_cast<uintptr_t>(scratch_dev) & 7u) != 0)
+        return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "gbc_weight_integral: scratch not 8-byte aligned");
+    double *table = static_cast<double *>(scratch_dev);
+    if (table != nullptr && std::fabs(S.v.gamma) <= kMaxGamma &&
+        aprict_b200_gbc_weight_integral_scratch_bytes(n_r, num_ang) > 0) {
+        k_gbc_height_table<<<kNodes * 32 / kGThreads, kGThreads, 0, st>>>(r_on_R_dev, n_r, table, num_z, S.v, tan_v);
+        // a CTA per radius where the radii alone fill the GPU
+        const int per_r = n_r >= 296 ? 1 : (num_ang + kGThreads - 1) / kGThreads;
+        k_gbc_weight_integ<<<dim3((unsigned)per_r, (unsigned)min(n_r, 65535)), kGThreads, 0, st>>>(
+            r_on_R_dev, n_r, out_dev, num_z, num_ang, S, tan_v, table);
+        return ab_cuda_check(cudaGetLastError(), "gbc_weight_integral launch");
+    }
     const dim3 grid((unsigned)((num_ang + kGThreads - 1) / kGThreads), (unsigned)min(n_r, 65535));
-    k_gbc_weight_integ<<<grid, kGThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        r_on_R_dev, n_r, out_dev, num_z, num_ang, S, (float)tan((double)cfg->soft_vartheta_v));
+    k_gbc_weight_integ<<<grid, kGThreads, 0, st>>>(r_on_R_dev, n_r, out_dev, num_z, num_ang, S, tan_v, nullptr);
     return ab_cuda_check(cudaGetLastError(), "gbc_weight_integral launch");
+}
+
+extern "C" int aprict_b200_gbc_weight_integral(const float *r_on_R_dev, int32_t n_r, double *out_dev, int32_t num_z,
+                                               int32_t num_ang, const aprict_backproject_config *cfg,
+                                               aprict_stream_t stream) {
+    return aprict_b200_gbc_weight_integral_scratch(r_on_R_dev, n_r, out_dev, num_z, num_ang, cfg, nullptr, stream);
 }
 
 extern "C" int aprict_b200_conebeam_spectral(void *spec_dev, int32_t n0, int32_t n1, int32_t n2, double multiplier,

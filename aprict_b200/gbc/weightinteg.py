@@ -29,10 +29,13 @@ def backproj_gbc_weight_integ_GPU(  # noqa: N802
     r = torch.from_numpy(np.ascontiguousarray(r_on_R, dtype=np.float32)).cuda()
     out = torch.zeros(len(r_on_R), dtype=torch.float64, device="cuda")
     cfg = config.contents
+    lib = _lib.lib()
+    nbytes = int(lib.aprict_b200_gbc_weight_integral_scratch_bytes(len(r_on_R), int(num_ang_samps)))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
     _lib.check(
-        _lib.lib().aprict_b200_gbc_weight_integral(
+        lib.aprict_b200_gbc_weight_integral_scratch(
             r.data_ptr(), len(r_on_R), out.data_ptr(), int(num_z_samps), int(num_ang_samps), _lib.ptr(cfg),
-            torch.cuda.current_stream().cuda_stream,
+            scratch.data_ptr() or None, torch.cuda.current_stream().cuda_stream,
         ),
         "gbc_weight_integral",
     )

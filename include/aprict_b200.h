@@ -350,6 +350,15 @@ APRICT_API int aprict_b200_gbc_weight_integral(const float *r_on_R_dev, int32_t 
                                                int32_t num_ang, const aprict_backproject_config *cfg,
                                                aprict_stream_t stream);
 
+/* The same with device scratch for a table of its inner sums, which replaces
+ * most of them by interpolation (error below the samples' rounding):
+ * aprict_b200_gbc_weight_integral_scratch_bytes bytes, 8-byte aligned (0 bytes
+ * or NULL: every inner sum is taken directly). */
+APRICT_API int64_t aprict_b200_gbc_weight_integral_scratch_bytes(int32_t n_r, int32_t num_ang);
+APRICT_API int aprict_b200_gbc_weight_integral_scratch(const float *r_on_R_dev, int32_t n_r, double *out_dev, int32_t num_z,
+                                                       int32_t num_ang, const aprict_backproject_config *cfg,
+                                                       void *scratch_dev, aprict_stream_t stream);
+
 /* In place on the (n0, n1, n2/2+1) complex64 rfftn spectrum of an (n0, n1,
  * n2) volume (axis 2 the cylinder axis): times multiplier * |k|, divided by
  * the softened Colsher k-factor of the polar angle (cone_angle in (0, pi);

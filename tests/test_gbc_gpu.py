@@ -104,6 +104,27 @@ def test_weight_integral_edges(r: np.ndarray, nz: int, na: int, soft: tuple) -> 
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6 * max(1.0, float(np.abs(want).max())))
 
 
+@pytest.mark.parametrize(("r", "nz", "na", "soft"), [
+    (np.linspace(0.0, 0.3, 40), 500, 700, SOFT),                       # interpolated inner sums
+    (np.linspace(0.0, 1.15, 60), 300, 500, SOFT),                      # past the sources: small ell summed directly
+    (np.linspace(0.3, 0.0, 40), 200, 700, SOFT),                       # radii out of order: outside the nodes
+    (np.zeros(1), 300, 20000, SOFT),                                   # no range of ell
+    (np.linspace(0.0, 0.3, 40), 500, 700, (0.22, 0.002, 0.45, 0.05)),  # a steep window: summed directly
+    (np.linspace(0.0, 0.3, 40), 500, 700, (0.22, 0.0065, 0.45, 0.05)),  # just below the steepest interpolated
+    (np.linspace(0.0, 0.3, 40), 300, 700, (2.0, 0.1, 1.7, 0.3)),
+])
+def test_weight_integral_table(r: np.ndarray, nz: int, na: int, soft: tuple) -> None:
+    """Calls large enough for the table of inner sums. The interpolation's error stays below 1e-7 (derived
+    beside the kernel); the gate is the direct sums'."""
+    cfg = fp.ConfigBackproject(fast_approx=True, backproj_weighting_preset=7, Z_on_val_factor_val=60.0,
+                               approx_mode_direct_raycast=True, soft_vartheta_v=soft[0],
+                               soft_vartheta_v_softspan=soft[1], soft_vartheta_h=soft[2],
+                               soft_vartheta_h_softspan=soft[3])
+    got = gbc.backproj_gbc_weight_integ_GPU(r, cfg, nz, na)
+    want = G.weight_integral(r.astype(np.float32), soft, nz, na)
+    np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6 * float(np.abs(want).max()))
+
+
 @pytest.mark.parametrize(("cone", "soft"), [(0.5, 0.05), (0.0, 0.0), (np.pi, 0.0), (1.2, 0.2)])
 def test_conebeam_filter_matches_oracle(cone: float, soft: float) -> None:
     rng = np.random.default_rng(int(cone * 10))
