@@ -77,6 +77,7 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
         _c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                  _c_void_p],
     ),
+    "aprict_b200_backproject_gbc_views": (_c_int, [_c_void_p] * 8 + [ctypes.c_uint32, _c_void_p, _c_void_p]),
     "aprict_b200_gbc_weight_integral_scratch_bytes": (ctypes.c_int64, [ctypes.c_int32, ctypes.c_int32]),
     "aprict_b200_gbc_weight_integral_scratch": (
         _c_int, [_c_void_p, ctypes.c_int32, _c_void_p, ctypes.c_int32, ctypes.c_int32, _c_void_p, _c_void_p, _c_void_p],

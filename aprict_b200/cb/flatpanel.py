@@ -734,9 +734,9 @@ def backproject(
         for it, first in _leading_slices(projs):
             specs, pd, dptr = _view_args(projs, it, first, data=p32)
             _lib.check(
-                _lib.lib().aprict_b200_backproject_gbc(
+                _lib.lib().aprict_b200_backproject_gbc_views(
                     specs, _lib.ptr(pd), dptr, _lib.ptr(vd), v32.data_ptr(), s32.data_ptr(),
-                    mptr, _lib.ptr(cfg), None, _stream(),
+                    mptr, _lib.ptr(cfg), projs._backproject_promise(False), None, _stream(),  # noqa: SLF001
                 ),
                 "backproject_gbc",
             )

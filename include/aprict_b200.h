@@ -342,6 +342,14 @@ APRICT_API int aprict_b200_backproject_gbc(const aprict_proj_spec *specs_dev, co
                                            const aprict_backproject_config *cfg, uint32_t *status_dev,
                                            aprict_stream_t stream);
 
+/* The same with what the caller knows of the views (APRICT_VIEWS_*, as in
+ * aprict_b200_backproject_views; Z factors play no part). */
+APRICT_API int aprict_b200_backproject_gbc_views(const aprict_proj_spec *specs_dev, const aprict_proj_desc *pd,
+                                                 const float *projs_dev, const aprict_vol_desc *vd, float *vol_dev,
+                                                 float *weightsum_dev, const float *multiplier_dev,
+                                                 const aprict_backproject_config *cfg, uint32_t views,
+                                                 uint32_t *status_dev, aprict_stream_t stream);
+
 /* out_dev[r] += the expected GBC weight sum at radius r_on_R_dev[r] (units of
  * R, increasing) over a perfect cylindrical locus sampled by num_z heights and
  * num_ang angles (get_GBC_weight_integ, CB_backproject.cu:1108-1168;

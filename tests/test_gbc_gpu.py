@@ -125,6 +125,27 @@ def test_weight_integral_table(r: np.ndarray, nz: int, na: int, soft: tuple) -> 
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6 * float(np.abs(want).max()))
 
 
+@pytest.mark.parametrize("nz", [9, 33, 65, 130, 257])
+@pytest.mark.parametrize("linear", [False, True])
+@pytest.mark.parametrize("soft", [SOFT, (0.1, 0.2, 0.45, 0.05), (1.7, 0.3, 0.45, 0.05)])
+def test_columns_match_oracle(nz: int, linear: bool, soft: tuple) -> None:
+    """The z-column kernel around its 32-voxel blocks, with blocks inside, across and past the vertical
+    window and the detector; windows wider than their angle and past pi/2."""
+    pg = _scan(m=70, h=60.0, nu=31, nv=40)  # odd: the grid's axis projects onto a column's middle
+    projs = np.random.default_rng(nz).random((70, 31, 40)).astype(np.float32)
+    shape, vw = (5, 11, nz), 0.9
+    cfg = fp.ConfigBackproject(fast_approx=True, backproj_weighting_preset=7, Z_on_val_factor_val=60.0,
+                               approx_mode_direct_raycast=True, approx_mode_bilinear_interpolate=linear, soft_vartheta_v=soft[0],
+                               soft_vartheta_v_softspan=soft[1], soft_vartheta_h=soft[2], soft_vartheta_h_softspan=soft[3])
+    v, ws = Volume.zeros(shape, voxwid=vw), Volume.zeros(shape, voxwid=vw)
+    fp.backproject(cfg, v, fp.ProjectionSet(pg, data=projs), secondary_volume=ws, block=True)
+    want, want_w = G.backproject_gbc(pg.to_proj_spec_array(), projs, shape, vw, v.corner, R=60.0, soft=soft, linear=linear,
+                                     ss=(1, 1, 1), mult=None)
+    assert np.linalg.norm(want) > 0
+    assert rel_l2(v.as_numpy(), want) <= 1e-5
+    assert rel_l2(ws.as_numpy(), want_w) <= 1e-5
+
+
 @pytest.mark.parametrize(("cone", "soft"), [(0.5, 0.05), (0.0, 0.0), (np.pi, 0.0), (1.2, 0.2)])
 def test_conebeam_filter_matches_oracle(cone: float, soft: float) -> None:
     rng = np.random.default_rng(int(cone * 10))
