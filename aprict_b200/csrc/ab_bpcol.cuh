@@ -70,34 +70,36 @@ struct ColSmem {
     float kcomp[kColWarps][32 * XB];
 };
 
-// ab_derive_bpview's FP64 forms for an upright view, by the same expressions
-// with the vanishing terms left out (the same values, a third of the work);
-// false for a degenerate view.
+// ab_derive_bpview's FP64 forms for an upright view with the vanishing terms
+// left out (a third of the work). The roundings are written out in the order in
+// which that function takes them: where a voxel lies exactly on the edge between
+// two pixels, the last bit of a form decides, and both kernels then choose alike.
+// False for a degenerate view.
 __device__ __forceinline__ bool derive_upright(const aprict_proj_spec &sp, ab_d3 c0, ab_bpview_d &o, double &Dn, double &uu,
                                                double &vv, ab_d3 &Ps, ab_d3 &c0s) {
     const ab_d3 s = ab_d3_of(sp.source_pos), P = ab_d3_of(sp.det_pos);
     const double ux = (double)sp.det_u.x, uy = (double)sp.det_u.y, vz = (double)sp.det_v.z;
-    const double nx = uy * vz, ny = -(ux * vz);
-    uu = ux * ux + uy * uy;
-    vv = vz * vz;
+    const double nx = __dmul_rn(uy, vz), ny = -__dmul_rn(ux, vz);
+    auto dot2 = [](double ax, double bx, double ay, double by) { return fma(ax, bx, __dmul_rn(ay, by)); };
+    uu = dot2(ux, ux, uy, uy);
+    vv = __dmul_rn(vz, vz);
     Ps = P - s;
     c0s = c0 - s;
-    Dn = Ps.x * nx + Ps.y * ny;
+    Dn = dot2(Ps.x, nx, Ps.y, ny);
     o = ab_bpview_d{};
     if (!(uu > 0.0 && vv > 0.0 && Dn != 0.0 && ab_finite3(s) && ab_finite3(P) && isfinite(uu) && isfinite(vv))) return false;
     const double hu = ((double)sp.nu - 1.0) * 0.5, hv = ((double)sp.nv - 1.0) * 0.5;
-    const double q = ux * Ps.x + uy * Ps.y, iu = 1.0 / uu, iv = 1.0 / vv;
-    o.nu[0] = (ux * Dn - nx * q) * iu + nx * hu;
-    o.nu[1] = (uy * Dn - ny * q) * iu + ny * hu;
-    o.nu[3] = o.nu[0] * c0s.x + o.nu[1] * c0s.y;
-    const double r = vz * Ps.z;
-    o.nv[0] = -(nx * r) * iv + nx * hv;
-    o.nv[1] = -(ny * r) * iv + ny * hv;
-    o.nv[2] = vz * Dn * iv;
-    o.nv[3] = o.nv[0] * c0s.x + o.nv[1] * c0s.y + o.nv[2] * c0s.z;
+    const double q = dot2(ux, Ps.x, uy, Ps.y), r = __dmul_rn(vz, Ps.z), iu = 1.0 / uu, iv = 1.0 / vv;
+    o.nu[0] = fma(fma(ux, Dn, -__dmul_rn(nx, q)), iu, __dmul_rn(nx, hu));
+    o.nu[1] = fma(fma(uy, Dn, -__dmul_rn(ny, q)), iu, __dmul_rn(ny, hu));
+    o.nu[3] = dot2(o.nu[0], c0s.x, o.nu[1], c0s.y);
+    o.nv[0] = fma(-__dmul_rn(nx, r), iv, __dmul_rn(nx, hv));
+    o.nv[1] = fma(-__dmul_rn(ny, r), iv, __dmul_rn(ny, hv));
+    o.nv[2] = __dmul_rn(__dmul_rn(vz, Dn), iv);
+    o.nv[3] = fma(o.nv[2], c0s.z, dot2(o.nv[0], c0s.x, o.nv[1], c0s.y));
     o.den[0] = nx;
     o.den[1] = ny;
-    o.den[3] = nx * c0s.x + ny * c0s.y;
+    o.den[3] = dot2(nx, c0s.x, ny, c0s.y);
     return true;
 }
 
@@ -173,7 +175,7 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
         const double fz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
         // the column's first voxel relative to the volume centre
         const double X = (ix + 0.5 + fx - 0.5 * P.n[0]) * P.vwd, Y = (iy + 0.5 + fy - 0.5 * P.n[1]) * P.vwd;
-        const double Z0 = (z0 + 0.5 + fz - 0.5 * P.n[2]) * P.vwd;
+        const double zi0 = z0 + 0.5 + fz - 0.5 * P.n[2], Z0 = zi0 * P.vwd;
         for (uint32_t v0 = 0; v0 < P.n_views; v0 += kChunk) {
             const int cn = (int)min((uint32_t)kChunk, P.n_views - v0);
             __syncthreads();
@@ -346,7 +348,7 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                         const int i = __float_as_int(t) - 0x4B400000 + crow;
                         float pv = ldg_if(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4, (unsigned)i < P.nv);
                         if (fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) > ra.w)
-                            pv = col_exact_row(sm.view[g0 + j].d, X, Y, fma((double)(lane + 32 * k), P.vwd, Z0), f, crow,
+                            pv = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f, crow,
                                                (int)P.nv, col, sv4);
                         const float rv = fabsf(f - coff);
                         if (P.sep > 0.f && rv > flatv && pv != 0.f) pv *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
@@ -382,7 +384,7 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                             const float f = k < 2 ? fo : fmaf((float)(k & ~1), s32, fo);
                             const float d = __fsub_rn(f, __fsub_rn(__fadd_rn(f, kMagic), kMagic));
                             if (!(in >> k & 1u) || fabsf(d) <= ra.w) continue;
-                            const float pe = col_exact_row(sm.view[g0 + j].d, X, Y, fma((double)(lane + 32 * k), P.vwd, Z0), f,
+                            const float pe = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f,
                                                            crow, (int)P.nv, col, sv4);
                             float q0, q1;
                             upk(pvp[k / 2], q0, q1);

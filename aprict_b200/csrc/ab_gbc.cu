@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kGThreads, 3) k_backproject_gbc_columns(const 
         const double oy = -0.5 + (0.5 + (isub / P.ssz) % P.ssy) / P.ssy;
         const double oz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
         const double X = (ix + 0.5 + ox - 0.5 * P.n[0]) * P.vwd, Y = (iy + 0.5 + oy - 0.5 * P.n[1]) * P.vwd;
-        const double Z0 = (z0 + 0.5 + oz - 0.5 * P.n[2]) * P.vwd;
+        const double zi0 = z0 + 0.5 + oz - 0.5 * P.n[2], Z0 = zi0 * P.vwd;
         // world position of the column's first voxel
         const float wx = (G.pos000[0] + (float)ix * P.voxwid) + (float)ox * P.voxwid;
         const float wy = (G.pos000[1] + (float)iy * P.voxwid) + (float)oy * P.voxwid;
@@ -636,9 +636,9 @@ __global__ void __launch_bounds__(kGThreads, 3) k_backproject_gbc_columns(const 
                                 upk(f, fa, fb);
                                 const ab_bpview_d &vd = sm.view[g0 + j].d;
                                 if (fabsf(da) > ra.z)
-                                    pa = col_exact_row(vd, X, Y, fma((double)(lane + 64 * k), P.vwd, Z0), fa, crow, (int)P.nv, col, sv4);
+                                    pa = col_exact_row(vd, X, Y, (zi0 + (double)(lane + 64 * k)) * P.vwd, fa, crow, (int)P.nv, col, sv4);
                                 if (fabsf(db) > ra.z)
-                                    pb = col_exact_row(vd, X, Y, fma((double)(lane + 64 * k + 32), P.vwd, Z0), fb, crow, (int)P.nv,
+                                    pb = col_exact_row(vd, X, Y, (zi0 + (double)(lane + 64 * k + 32)) * P.vwd, fb, crow, (int)P.nv,
                                                        col, sv4);
                             }
                             pv = pk(pa, pb);
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(kGThreads, 3) k_backproject_gbc_columns(const 
                         } else {
                             const float t = __fadd_rn(f, kMagic);
                             if (fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) > ra.z)
-                                pv = col_exact_row(sm.view[g0 + j].d, X, Y, fma((double)(lane + 32 * k), P.vwd, Z0), f, crow,
+                                pv = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f, crow,
                                                    (int)P.nv, col, sv4);
                             else if ((unsigned)(__float_as_int(t) - 0x4B400000 + crow) < P.nv)
                                 pv = __ldg(reinterpret_cast<const float *>(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4));

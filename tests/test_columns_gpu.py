@@ -142,3 +142,17 @@ def test_batch_of_upright_and_tilted_scans(mode: str) -> None:
     ScanBatch(vols, [fp.ProjectionSet(g, data=d) for g, d in zip(pgs, datas)]).backproject(cfg, block=True)
     for s, g, d, v in zip(shapes, pgs, datas, vols):
         assert rel_l2(v.as_numpy(), _run(mode, g, d, s)) <= 1e-6
+
+
+@pytest.mark.parametrize(("shape", "nu", "nv"), [((20, 22, 33), 31, 40), ((21, 19, 64), 30, 41), ((21, 19, 131), 30, 40)])
+@pytest.mark.parametrize("mode", ["nearest", "raycast"])
+def test_exact_ties_fall_as_in_the_bricks(mode: str, shape: tuple, nu: int, nv: int) -> None:
+    """Odd heights on an even detector put the mid plane on the edge between two rows in every view, odd widths the
+    axis between two columns: the last bit of the FP64 forms decides, the same one in both kernels. FP32 sums agree to
+    1e-6; a voxel-view on the other side changes its voxel by a pixel's difference over 70 views, 1e-3 of the largest."""
+    for vw in (1.0, 0.9):
+        pg = circular(70, 160, 120, 0.913, nu, nv, theta0=0.3)
+        data = _data(pg, 11)
+        got, bricks = _run(mode, pg, data, shape, vw=vw), _run(mode, pg, data, shape, views=2, vw=vw)
+        assert np.abs(got - bricks).max() <= 1e-5 * np.abs(bricks).max()
+        assert rel_l2(got, bricks) <= 1e-6

@@ -146,6 +146,22 @@ def test_columns_match_oracle(nz: int, linear: bool, soft: tuple) -> None:
     assert rel_l2(ws.as_numpy(), want_w) <= 1e-5
 
 
+@pytest.mark.parametrize(("shape", "nu", "nv"), [((20, 22, 33), 31, 40), ((21, 19, 64), 30, 41)])
+def test_exact_ties_fall_as_in_the_general_kernel(shape: tuple, nu: int, nv: int) -> None:
+    """As the columns' test of the same name: mid plane or axis between two pixels in every view of a circular scan."""
+    pg = _scan(m=70, h=0.0, nu=nu, nv=nv)
+    projs = np.random.default_rng(3).random((70, nu, nv)).astype(np.float32)
+    out = []
+    for views in (1, 2):
+        v, ws = Volume.zeros(shape, voxwid=0.9), Volume.zeros(shape, voxwid=0.9)
+        ps = fp.ProjectionSet(pg, data=projs)
+        ps._backproject_promise = lambda needs_z, views=views: views  # noqa: SLF001
+        fp.backproject(_cfg(False), v, ps, secondary_volume=ws, block=True)
+        out.append(v.as_numpy())
+    assert np.linalg.norm(out[1]) > 0
+    assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[1]).max()
+
+
 @pytest.mark.parametrize(("cone", "soft"), [(0.5, 0.05), (0.0, 0.0), (np.pi, 0.0), (1.2, 0.2)])
 def test_conebeam_filter_matches_oracle(cone: float, soft: float) -> None:
     rng = np.random.default_rng(int(cone * 10))
