@@ -29,11 +29,16 @@
 // warp instructions per 32 voxel-views against 21 of the brick kernel's z-lane
 // path before it, issue 54 %, L1 wavefronts 60 %). Measured there, four CTAs per
 // SM: nearest 4.93 -> 3.11 ms (F order 14.8 -> 3.3 ms: its lanes gathered 32
-// pixel columns), direct raycast 13.8 -> 3.1 ms, on a helical scan 12.4 -> 6.5 ms
-// (columns cut by the detector's edges); 64^3 x 90 views 72 -> 55 us; bilinear
-// on 210 x 190 x 150 x 200 views 2.06 -> 1.73 ms. Three CTAs at 80 registers, no
-// spills: 3.6 ms. Blocks across the detector's edge are gathered under a
-// predicate (a branch around the gather: 7.6 ms on the helical scan).
+// pixel columns), direct raycast 13.8 -> 3.1 ms; 64^3 x 90 views 72 -> 55 us;
+// bilinear on 210 x 190 x 150 x 200 views 2.06 -> 1.73 ms. Three CTAs at 80
+// registers, no spills: 3.6 ms.
+//
+// Columns cut by the detector's edges (helical scans; 256^3 x 180 views, one
+// turn): nearest 7.2 -> 3.8 ms, direct raycast 6.3 -> 2.8 ms. Their blocks are
+// gathered under a predicate (a branch around the gather: twice the time), blocks
+// inside four at a time, and their close rows settled together with the others'
+// (a call in each block, around which the column's registers spill: 5.2 and 3.6
+// ms, and 1.62 instead of 1.57 ms on the circular scan, which has no such column).
 #pragma once
 
 #include "ab_bpbrick.cuh"
@@ -325,19 +330,20 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                         acc2[k] = fma2(pvp[k], w2, acc2[k]);
                         pvp[k] = pk(pa, pb);
                     };
-                    // one block across the flat box's or the detector's edge
+                    // one block across the flat box's or the detector's edge (or off it: nothing is
+                    // gathered), without branches; a lane past the volume's top gathers along where
+                    // its row exists and is never written
                     auto edge_block = [&](int k) -> float {
-                        // (a lane past the volume's top gathers along where its row exists; never written)
-                        if (!((in | across) >> k & 1u)) return 0.f;  // warp-uniform
+                        const bool on = (in | across) >> k & 1u;
                         const float fo = (k & 1) ? a + s32 : a;
                         const float f = fminf(fmaxf(k < 2 ? fo : fmaf((float)(k & ~1), s32, fo), -2097152.f), 2097152.f);
                         if constexpr (BILIN) {
                             const float fl = floorf(f), fy = f - fl;
                             const int j0 = (int)fl + crow;
                             const float *p = reinterpret_cast<const float *>(col + 4ull * 0x4B400000ull) + (j0 - crow);
-                            const bool r0 = (unsigned)j0 < P.nv, r1 = (unsigned)(j0 + 1) < P.nv, c0 = rb.w & 1u, c1 = rb.w & 2u;
-                            const float v00 = r0 && c0 ? __ldg(p) : 0.f, v01 = r1 && c0 ? __ldg(p + 1) : 0.f;
-                            const float v10 = r0 && c1 ? __ldg(p + P.su) : 0.f, v11 = r1 && c1 ? __ldg(p + P.su + 1) : 0.f;
+                            const bool r0 = on && (unsigned)j0 < P.nv, r1 = on && (unsigned)(j0 + 1) < P.nv, c0 = rb.w & 1u, c1 = rb.w & 2u;
+                            const float v00 = ldg_if((uint64_t)p, r0 && c0), v01 = ldg_if((uint64_t)(p + 1), r1 && c0);
+                            const float v10 = ldg_if((uint64_t)(p + P.su), r0 && c1), v11 = ldg_if((uint64_t)(p + P.su + 1), r1 && c1);
                             const float t1 = v00 * (1.f - ra.w) + v10 * ra.w, t2 = v01 * (1.f - ra.w) + v11 * ra.w;
                             float pv = t1 * (1.f - fy) + t2 * fy;
                             const float rv = fabsf(f - coff);
@@ -346,10 +352,8 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                         }
                         const float t = __fadd_rn(f, kMagic);
                         const int i = __float_as_int(t) - 0x4B400000 + crow;
-                        float pv = ldg_if(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4, (unsigned)i < P.nv);
-                        if (fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) > ra.w)
-                            pv = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f, crow,
-                                               (int)P.nv, col, sv4);
+                        float pv = ldg_if(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4, on && (unsigned)i < P.nv);
+                        tie = fmaxf(tie, on ? fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) : 0.f);
                         const float rv = fabsf(f - coff);
                         if (P.sep > 0.f && rv > flatv && pv != 0.f) pv *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
                         return pv;
@@ -358,11 +362,23 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
 #pragma unroll
                         for (int k = 0; k < XB / 2; ++k) inner_pair(k);
                     } else {
+                        // four blocks at a time where all lie inside, so that the rest of a column cut by
+                        // the detector's edge keeps its gathers together
+                        constexpr int kPart = XB < 4 ? XB : 4;
+                        constexpr unsigned kFull = (1u << kPart) - 1u;
 #pragma unroll
-                        for (int k = 0; k < XB / 2; ++k) {  // warp-uniform branches
-                            if ((in >> (2 * k) & 3u) == 3u) {
-                                inner_pair(k);
-                            } else {
+                        for (int h = 0; h < XB; h += kPart) {  // warp-uniform branches
+                            if ((in >> h & kFull) == kFull) {
+#pragma unroll
+                                for (int k = h / 2; k < (h + kPart) / 2; ++k) inner_pair(k);
+                                continue;
+                            }
+#pragma unroll
+                            for (int k = h / 2; k < (h + kPart) / 2; ++k) {
+                                if ((in >> (2 * k) & 3u) == 3u) {
+                                    inner_pair(k);
+                                    continue;
+                                }
                                 if (!BILIN) {
                                     acc2[k] = fma2(pvp[k], w2, acc2[k]);
                                     pvp[k] = pk(0.f, 0.f);
@@ -378,17 +394,23 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                         }
                     }
                     if (!BILIN && tie > ra.w) {  // some row of this lane is too close to call in FP32
-#pragma unroll
+#pragma unroll 1
                         for (int k = 0; k < XB; ++k) {
                             const float fo = (k & 1) ? a + s32 : a;
                             const float f = k < 2 ? fo : fmaf((float)(k & ~1), s32, fo);
-                            const float d = __fsub_rn(f, __fsub_rn(__fadd_rn(f, kMagic), kMagic));
-                            if (!(in >> k & 1u) || fabsf(d) <= ra.w) continue;
-                            const float pe = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f,
-                                                           crow, (int)P.nv, col, sv4);
-                            float q0, q1;
-                            upk(pvp[k / 2], q0, q1);
-                            pvp[k / 2] = (k & 1) ? pk(q0, pe) : pk(pe, q1);
+                            const float fc = fminf(fmaxf(f, -2097152.f), 2097152.f);
+                            const float d = __fsub_rn(fc, __fsub_rn(__fadd_rn(fc, kMagic), kMagic));
+                            if (!((in | across) >> k & 1u) || fabsf(d) <= ra.w) continue;
+                            float pe = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, fc,
+                                                     crow, (int)P.nv, col, sv4);
+                            const float rv = fabsf(fc - coff);
+                            if (P.sep > 0.f && rv > flatv && pe != 0.f) pe *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
+#pragma unroll
+                            for (int m = 0; m < XB / 2; ++m) {  // registers: the index has to be constant
+                                float q0, q1;
+                                upk(pvp[m], q0, q1);
+                                pvp[m] = pk(k == 2 * m ? pe : q0, k == 2 * m + 1 ? pe : q1);
+                            }
                         }
                     }
                 }

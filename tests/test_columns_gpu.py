@@ -156,3 +156,18 @@ def test_exact_ties_fall_as_in_the_bricks(mode: str, shape: tuple, nu: int, nv: 
         got, bricks = _run(mode, pg, data, shape, vw=vw), _run(mode, pg, data, shape, views=2, vw=vw)
         assert np.abs(got - bricks).max() <= 1e-5 * np.abs(bricks).max()
         assert rel_l2(got, bricks) <= 1e-6
+
+
+@pytest.mark.parametrize("pitch", [0.3, 1.0, 3.0])
+@pytest.mark.parametrize("mode", ["nearest-taper", "raycast", "bilinear-taper"])
+def test_columns_cut_by_the_detector(mode: str, pitch: float) -> None:
+    """Helical columns of 2, 4 and 8 blocks, of which each view sees a few: all inside, four inside, pairs, edges."""
+    for nz in (60, 120, 250):
+        shape = (9, 10, nz)
+        pg = geometry.helical_scan(n_views=70, R=300.0, L_minus_R=200.0, pix_at_iso=0.83, nu=21, nv=150, pitch=pitch, theta_start=0.31)
+        data = _data(pg, nz)
+        want = _oracle(mode, pg, data, shape)
+        assert np.linalg.norm(want) > 0
+        got = _run(mode, pg, data, shape)
+        assert rel_l2(got, want) <= 1e-5
+        assert rel_l2(_run(mode, pg, data, shape, views=2), got) <= (1e-5 if "bilinear" in mode else 1e-6)
