@@ -434,8 +434,9 @@ __global__ void __launch_bounds__(kGThreads, BILIN ? 3 : 4) k_backproject_gbc_z(
 // (fast), past the window (weight 0: skipped) or neither. A fast voxel-view
 // is then ell^3 A / h^3 from one reciprocal square root, the row, the gathers
 // and two fmas, on pairs of voxels. Measured, 198^3 x 360 views x 256^2
-// bilinear: 13.0 ms (k_backproject_gbc_z) -> 6.4 ms, 4.7e9 warp instructions against
-// 1.2e10; 7.8 ms with the window's band left to the per-voxel branch.
+// bilinear: 13.0 ms (k_backproject_gbc_z) -> 5.6 ms, 4.7e9 warp instructions against
+// 1.2e10, at 4 CTAs per SM (64 registers; 6.4 ms at 3, 7.9 ms at 2; 7.8 ms at 3 with
+// the window's band left to the per-voxel branch).
 struct GbcView {
     ab_bpview_d d;
     float sx, sy, sz, inv_ls;  // source, 1 / |(sx, sy)|
@@ -460,7 +461,7 @@ struct GbcColSmem {
 };
 
 template <bool BILIN>
-__global__ void __launch_bounds__(kGThreads, 3) k_backproject_gbc_columns(const ab_bp::BPParams P, const GbcParams G,
+__global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const ab_bp::BPParams P, const GbcParams G,
                                                                           float tan_flat, float tan_zero, int clamped) {
     using namespace ab_bp;
     extern __shared__ __align__(16) unsigned char smem_raw[];
