@@ -17,8 +17,9 @@
 // load, one 16-byte gather and 4 fmas.
 // Bound: the L1's 128 bytes per clock (4 B per voxel, view and slice).
 // Measured, 64 slices 512^2 x 720 views x 1024: 24 ms (every slice by itself, one
-// persistent launch) -> 3.4 ms; L1 data path 60 %, the rest gather latency at 16
-// warps per SM (32 accumulators and 32 gathered values a thread).
+// persistent launch) -> 3.4 ms with 8 voxels per thread and 16 warps per SM; with 4
+// and 32, as here, the whole reconstruction of the stack takes 4.6 ms instead of
+// 5.1 (the gathers' latency wants the warps more than the shared loads the reuse).
 // Accumulation as in bp_brick: FP32 over a chunk of views, the chunks under
 // Kahan's compensation (totals and compensations in shared memory).
 #include <cuda_runtime.h>
@@ -29,9 +30,9 @@ namespace {
 
 using namespace ab_bp;
 
-constexpr int kVox = 8;       // voxels per thread
+constexpr int kVox = 4;       // voxels per thread
 constexpr int kMaxSlices = 64;
-constexpr int kEntries = 2048;  // (view, voxel) entries per table fill
+constexpr int kEntries = 1024;  // (view, voxel) entries per table fill
 constexpr int kViews = 64;      // views per coefficient chunk (and per FP32 partial sum)
 constexpr int kTileY = 16;
 
@@ -52,7 +53,7 @@ struct SliceSmem {
 
 // LS: lanes per voxel (4 LS >= slices).
 template <int LS>
-__global__ void __launch_bounds__(kThreads, 2) k_backproject_slices(const __grid_constant__ SliceArgs A) {
+__global__ void __launch_bounds__(kThreads, 4) k_backproject_slices(const __grid_constant__ SliceArgs A) {
     constexpr int kGroups = 32 / LS;             // voxel groups per warp
     constexpr int kTile = kWarps * kGroups * kVox;  // voxels per CTA
     constexpr int kStep = kEntries / kTile;      // views per table fill
