@@ -169,9 +169,9 @@ def fbp_fan_circ_batch(
     for p in projs:
         if id(p.proj_geom) not in by_id:
             by_id[id(p.proj_geom)] = fan_geometry(p.proj_geom)
-    geo = [by_id[id(p.proj_geom)] for p in projs]
+    geo = list(by_id.values())
     m = projs[0].proj_geom.num_projs
-    if any(not np.allclose(g, geo[0]) for g in geo) or any(p.proj_geom.num_projs != m for p in projs):
+    if any(not np.allclose(g, geo[0]) for g in geo) or any(p.proj_specs.size != m for p in projs):
         msg = "batched fan FBP needs one fan geometry and view count for every slice"
         raise NotImplementedError(msg)
     R, L, pixwid, nu, nv = geo[0]  # noqa: N806
