@@ -119,6 +119,14 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
     "aprict_b200_batch_plan": (_c_int, [_c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, ctypes.c_size_t]),
     "aprict_b200_batch_run": (_c_int, [_c_void_p, _c_void_p, _c_void_p]),
     "aprict_b200_batch_run_static": (_c_int, [_c_void_p, _c_void_p]),
+    "aprict_b200_project_forbild_scratch_bytes": (ctypes.c_int64, [ctypes.c_int64, ctypes.c_int64]),
+    "aprict_b200_project_forbild_scratch": (
+        _c_int,
+        [
+            _c_void_p, _c_void_p, _c_void_p, _c_void_p, ctypes.c_int64, ctypes.c_float, ctypes.c_uint32,
+            ctypes.c_uint32, _c_int, _c_void_p, _c_void_p, _c_void_p, ctypes.c_int64, _c_void_p,
+        ],
+    ),
     "aprict_b200_project_forbild": (
         _c_int,
         [

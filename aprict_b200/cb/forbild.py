@@ -78,12 +78,16 @@ def project_shapes(config: object, volume: object, projs: object) -> None:
     else:
         mode = 0
     counter = projs.out_of_mem_counter
+    lib = _lib.lib()
+    nbytes = int(lib.aprict_b200_project_forbild_scratch_bytes(int(projs.proj_specs.shape[-1]), comp.n))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=comp.dev.device)
     for it, first in _leading_slices(projs):
         specs, pd, dptr = _view_args(projs, it, first)
         _lib.check(
-            _lib.lib().aprict_b200_project_forbild(
+            lib.aprict_b200_project_forbild_scratch(
                 specs, _lib.ptr(pd), dptr, comp.dev.data_ptr(), comp.n, float(cfg["multiply_before_adding"]),
-                int(cfg["ssu"]), int(cfg["ssv"]), mode, counter.data_ptr(), None, _stream(),
+                int(cfg["ssu"]), int(cfg["ssv"]), mode, counter.data_ptr(), None, scratch.data_ptr() or None, nbytes,
+                _stream(),
             ),
             "project (FORBILD)",
         )

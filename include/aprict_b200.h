@@ -449,6 +449,17 @@ APRICT_API int aprict_b200_project_forbild(const aprict_proj_spec *specs_dev, co
                                            float multiply_before_adding, uint32_t ssu, uint32_t ssv, int mode,
                                            uint32_t *overflow_dev, uint32_t *status_dev, aprict_stream_t stream);
 
+/* The same with device scratch for the per-(view, shape) records (16-byte
+ * aligned; aprict_b200_project_forbild_scratch_bytes for all views at once, at
+ * most 256 MB; with less than one view's the call takes stream-ordered memory,
+ * as above). */
+APRICT_API int64_t aprict_b200_project_forbild_scratch_bytes(int64_t n_views, int64_t n_shapes);
+APRICT_API int aprict_b200_project_forbild_scratch(const aprict_proj_spec *specs_dev, const aprict_proj_desc *projs,
+                                                   float *projs_dev, const aprict_quadric *shapes_dev, int64_t n_shapes,
+                                                   float mba, uint32_t ssu, uint32_t ssv, int mode, uint32_t *overflow_dev,
+                                                   uint32_t *status_dev, void *scratch_dev, int64_t scratch_bytes,
+                                                   aprict_stream_t stream);
+
 /* ---- SIRT (reference mode) ----
  * One iteration of SIRT_flatpanel (sirt_vram.py:130-152) as two launches on
  * the stream: r = b - A x (fused residual), then x += M (.) B r with cfg_bp
