@@ -121,7 +121,11 @@ AB_HD ab_d3 ab_to_grid(const ab_grid<Off> &g, ab_d3 p) {
 // plane c == 0 misses and one in c == n hits the last layer.
 //
 // ab_siddon_setup prepares the traversal state (in FP64, then rounded to the
-// FP32 stepping quantities); ab_siddon runs it with a visitor. Both return
+// FP32 stepping quantities), a tenth of a short ray's instructions: with the
+// range-checked reciprocal and root, a minimum and maximum per axis and the
+// counts' fix-up loops entered by every ray 128^3 x 90 views took 1.167 ms instead
+// of 1.142 (the views' own conversions kept in shared memory: 1.19 ms, the CTA
+// waits for them). ab_siddon runs it with a visitor. Both return
 // false when the segment misses the grid or its input is not finite (*bad is
 // set for non-finite input).
 template <typename Off>
@@ -140,28 +144,35 @@ AB_HD bool ab_siddon_setup(ab_d3 o, ab_d3 e, const int n[3], const Off stride[3]
         return false;
     }
     const double od[3] = {o.x, o.y, o.z};
-    const double dd[3] = {e.x - o.x, e.y - o.y, e.z - o.z};
+    double dd[3] = {e.x - o.x, e.y - o.y, e.z - o.z};
     double a_in = 0.0, a_out = 1.0;
-    double inv[3];  // 1 / dd (correctly rounded), reused below instead of divisions
+    double inv[3];  // 1 / dd, reused below instead of divisions
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         inv[a] = 0.0;
-        if (dd[a] == 0.0) {
+        if (fabs(dd[a]) < 1e-300) {  // parallel to the axis's planes
             if (!(od[a] > 0.0 && od[a] <= (double)n[a])) return false;
+            dd[a] = 0.0;
         } else {
 #if defined(__CUDA_ARCH__)
-            inv[a] = __drcp_rn(dd[a]);
+            inv[a] = ab_rcp_h3(dd[a]);
 #else
             inv[a] = 1.0 / dd[a];
 #endif
             const double t0 = (0.0 - od[a]) * inv[a];
             const double t1 = ((double)n[a] - od[a]) * inv[a];
-            a_in = fmax(a_in, fmin(t0, t1));
-            a_out = fmin(a_out, fmax(t0, t1));
+            const bool pos = dd[a] > 0.0;  // then t0 < t1
+            a_in = fmax(a_in, pos ? t0 : t1);
+            a_out = fmin(a_out, pos ? t1 : t0);
         }
     }
     if (!(a_in < a_out)) return false;
-    const double len = sqrt(dd[0] * dd[0] + dd[1] * dd[1] + dd[2] * dd[2]);
+    const double len2 = dd[0] * dd[0] + dd[1] * dd[1] + dd[2] * dd[2];
+#if defined(__CUDA_ARCH__)
+    const double len = len2 > 0.0 ? ab_sqrt_h3(len2) : 0.0;
+#else
+    const double len = sqrt(len2);
+#endif
 
     int stp[3];
     float t0f[3], dtf[3], texit[3];
@@ -169,12 +180,14 @@ AB_HD bool ab_siddon_setup(ab_d3 o, ab_d3 e, const int n[3], const Off stride[3]
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const double p = od[a] + a_in * dd[a];
-        int i;
-        if (dd[a] > 0.0) {
-            i = (int)floor(p);
-        } else {
-            i = (int)ceil(p) - 1;
-        }
+        const bool pos = dd[a] > 0.0;
+        // floor(p), or ceil(p) - 1 = -floor(-p) - 1 against the axis
+#if defined(__CUDA_ARCH__)
+        const int f = __double2int_rd(pos ? p : -p);
+#else
+        const int f = (int)floor(pos ? p : -p);
+#endif
+        int i = pos ? f : -f - 1;
         i = i < 0 ? 0 : (i >= n[a] ? n[a] - 1 : i);
         off += (Off)i * stride[a];
         if (dd[a] == 0.0) {
@@ -183,9 +196,8 @@ AB_HD bool ab_siddon_setup(ab_d3 o, ab_d3 e, const int n[3], const Off stride[3]
             dtf[a] = 0.f;
             texit[a] = INFINITY;
         } else {
-            const bool pos = dd[a] > 0.0;
             stp[a] = pos ? 1 : -1;
-            const double b = pos ? (double)(i + 1) : (double)i;
+            const double b = (double)(pos ? i + 1 : i);
             const double ab = (b - od[a]) * inv[a];
             t0f[a] = (float)((ab - a_in) * len);
             dtf[a] = (float)(len * fabs(inv[a]));
@@ -293,6 +305,7 @@ AB_HD int ab_axis_count(float t0, float dt, float tend, bool &ok) {
     const float q = (tend - t0) / dt;
 #endif
     int k = q < 1.f ? 1 : (q > 16777216.f ? 16777216 : (int)ceilf(q));
+    if (fmaf((float)(k - 1), dt, t0) < tend && fmaf((float)k, dt, t0) >= tend) return k;  // almost always
     for (int it = 0; it < 8 && k > 1 && fmaf((float)(k - 1), dt, t0) >= tend; ++it) --k;
     for (int it = 0; it < 8 && fmaf((float)k, dt, t0) < tend; ++it) ++k;
     if (!(fmaf((float)(k - 1), dt, t0) < tend && fmaf((float)k, dt, t0) >= tend)) ok = false;
