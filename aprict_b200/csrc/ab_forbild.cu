@@ -332,7 +332,7 @@ __device__ bool footprint(const ViewGeom &g, const aprict_quadric &q, double &u0
         const double den = ab_dot(r, g.n) * (g.Dn > 0 ? 1.0 : -1.0);
         if (!(den > 0.0)) return false;
         const double sden = ab_dot(r, g.n);
-        const double fu = ab_dot(g.Au, r) / sden, fv = ab_dot(g.Av, r) / sden;
+        const double is = 1.0 / sden, fu = ab_dot(g.Au, r) * is, fv = ab_dot(g.Av, r) * is;
         u0 = fmin(u0, fu);
         u1 = fmax(u1, fu);
         v0 = fmin(v0, fv);
@@ -348,8 +348,9 @@ __device__ void make_forms(const ViewGeom &g, const aprict_quadric &q, QView &o)
     const ab_d3 r = ab_d3{q.c[0], q.c[1], q.c[2]} - g.s;
     const double den = ab_dot(r, g.n);
     if (!(den * g.Dn > 0.0)) return;  // the centre is not in front of the source
-    o.uc = ab_dot(g.Au, r) / den;
-    o.vc = ab_dot(g.Av, r) / den;
+    const double iden = 1.0 / den;
+    o.uc = ab_dot(g.Au, r) * iden;
+    o.vc = ab_dot(g.Av, r) * iden;
     const int n = q.kind == 1 ? 3 : 2;
     double c[3], w0[3], wu[3], wv[3];  // direction at the centre; o x d there and its steps
     for (int k = 0; k < 3; ++k) c[k] = fma(o.dv[k], o.vc, fma(o.du[k], o.uc, o.d0[k]));
@@ -385,11 +386,12 @@ __device__ void make_forms(const ViewGeom &g, const aprict_quadric &q, QView &o)
     const double size = dot(o.d0, o.d0, n);
     o.a_min = 1e-9 * fmax(o.A[0], size);
     // t of a point is its depth over the detector's; the solid lies in its box
+    const double iDn = 1.0 / g.Dn;
     double t0 = 1e300, t1 = -1e300;
     for (int k = 0; k < 8; ++k) {
         const ab_d3 x{q.c[0] + ((k & 4) ? q.bb_half[0] : -q.bb_half[0]), q.c[1] + ((k & 2) ? q.bb_half[1] : -q.bb_half[1]),
                       q.c[2] + ((k & 1) ? q.bb_half[2] : -q.bb_half[2])};
-        const double t = ab_dot(x - g.s, g.n) / g.Dn;
+        const double t = ab_dot(x - g.s, g.n) * iDn;
         t0 = fmin(t0, t);
         t1 = fmax(t1, t);
     }
