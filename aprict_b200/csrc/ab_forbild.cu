@@ -58,7 +58,8 @@ struct QView {
     // cbb b^2, B linear. At the centre o x d = 0, so disc loses nothing to the
     // cancellation of B^2 and A C.
     double uc, vc, A[6], B[3], disc[6];
-    double a_min;  // below it (a ray along a cylinder's axis) the general solver runs
+    double a_min;     // below it (a ray along a cylinder's axis, a centre beside the source) the general solver runs
+    double disc_min;  // (negative) what a discriminant of 0 may come out as: below it the ray misses
     int fast;
     int between;  // every point of the solid lies strictly between the source and the detector: 0 < t < 1
 };
@@ -298,6 +299,7 @@ namespace {
 
 struct ViewGeom {
     ab_d3 s, P, U, V, n, Au, Av, D0;  // D0 = P - s - U hu - V hv
+    double hu, hv;                    // the centre's pixel index
     double s_n;                       // s . n
     double Dn;
 };
@@ -310,7 +312,7 @@ __device__ void view_geom(const aprict_proj_spec &sp, ViewGeom &g) {
     g.n = ab_cross(g.U, g.V);
     const ab_d3 Ps = g.P - g.s;
     g.Dn = ab_dot(Ps, g.n);
-    const double hu = ((double)sp.nu - 1.0) * 0.5, hv = ((double)sp.nv - 1.0) * 0.5;
+    const double hu = g.hu = ((double)sp.nu - 1.0) * 0.5, hv = g.hv = ((double)sp.nv - 1.0) * 0.5;
     // pixel index of a point x: (Au.(x-s)) / ((x-s).n), same for v
     g.Au = (g.U * g.Dn - g.n * ab_dot(g.U, Ps)) * (1.0 / ab_dot(g.U, g.U)) + g.n * hu;
     g.Av = (g.V * g.Dn - g.n * ab_dot(g.V, Ps)) * (1.0 / ab_dot(g.V, g.V)) + g.n * hv;
@@ -382,9 +384,16 @@ __device__ void make_forms(const ViewGeom &g, const aprict_quadric &q, QView &o)
     o.disc[3] = o.A[3] - dot(wu, wu, 3);
     o.disc[4] = o.A[4] - 2.0 * dot(wu, wv, 3);
     o.disc[5] = o.A[5] - dot(wv, wv, 3);
-    // A's terms cancel towards a cylinder's axis: 1e-9 of their size is still good to 1e-7
+    // A's terms cancel towards a cylinder's axis, and for a centre beside the source, whose
+    // direction is far longer than a pixel's: 1e-6 of their size is still good to 1e-10
     const double size = dot(o.d0, o.d0, n);
-    o.a_min = 1e-9 * fmax(o.A[0], size);
+    o.a_min = 1e-6 * fmax(o.A[0], size);
+    // Rounding of disc over the detector: its terms are at most S^2 and (|o| S)^2, S =
+    // |c| + |du| max |a| + |dv| max |b|, and coefficients and sum are good to some 30
+    // units of 2^-53 of them. A ray along a cylinder's axis has A = disc = 0: the sign of
+    // a disc this small says nothing, and A has to be asked first.
+    const double am = fabs(o.uc - g.hu) + g.hu + 1.0, bm = fabs(o.vc - g.hv) + g.hv + 1.0;
+    o.disc_min = -1e-14 * (1.0 + dot(o.o, o.o, n)) * fma(o.A[5], bm * bm, fma(o.A[3], am * am, o.A[0]));
     // t of a point is its depth over the detector's; the solid lies in its box
     const double iDn = 1.0 / g.Dn;
     double t0 = 1e300, t1 = -1e300;
@@ -552,7 +561,7 @@ __device__ __noinline__ bool ray_interval_general(const QView &q, double fu, dou
 }
 
 // The same for ellipsoids and cylinders from their polynomial record: a ray
-// that misses the solid ends after the discriminant, and the cylinder's caps
+// that misses the solid by more than rounding ends after the discriminant, and the cylinder's caps
 // and the clip planes divide only where they cut the interval found so far.
 // A miss costs 7 FP64 operations (the direction, A, B and C first: some 25), a
 // hit's two roots no division: 240 views x 1024^2 of 100 clipped quadrics 15.4 ->
@@ -561,7 +570,7 @@ __device__ __forceinline__ bool ray_interval(const QView &q, double fu, double f
     if (!q.fast) return ray_interval_general(q, fu, fv, lo, hi);
     const double a = fu - q.uc, b = fv - q.vc;
     const double disc = form6(q.disc, a, b);
-    if (!(disc > 0.0)) return false;
+    if (!(disc > q.disc_min)) return false;
     const double A = form6(q.A, a, b);
     if (!(A > q.a_min)) return ray_interval_general(q, fu, fv, lo, hi);
     // a chord below 1e-10 of the solid's size is under the discriminant's own rounding

@@ -232,3 +232,55 @@ def test_gpu_ray_forms_at_their_edges(mode_kw: dict, mode: int, alone: bool) -> 
         top = np.abs(want).max()
         assert np.abs(got - want).max() <= 2e-5 * max(top, 1e-30), sh["type"]
         assert rel_l2(got, want) <= 1e-6 if top > 0 else not got.any()
+
+
+def _end_on(n: int, theta: float, axis: str) -> np.ndarray:
+    """Cylinders of radius 6 along the central ray of the view at ``theta``, their axes up to 3 off it: the ray lies
+    inside, parallel to the axis."""
+    rng = np.random.default_rng(31)
+    sh = np.zeros(n, S.forbild_shape)
+    for k in range(n):
+        rec = sh[k]
+        rec["type"], rec["rho"], rec["r"], rec["l"] = {"x": 7, "y": 8, "free": 6}[axis], 0.7, 6.0, 40.0
+        rec["x"], rec["y"], rec["z"] = rng.uniform(-3, 3, 3)
+        rec["axis"] = (np.cos(theta), np.sin(theta), 0.0)
+    return sh
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize(("theta", "axis"), [(0.0, "x"), (0.5 * np.pi, "y"), (0.0, "free"), (0.7, "free")])
+@pytest.mark.parametrize("nu", [65, 64])
+def test_gpu_cylinders_seen_end_on(theta: float, axis: str, nu: int) -> None:
+    """Rays along a cylinder's axis have A = 0 and a discriminant of 0, either sign by rounding: inside they get the
+    whole chord. Every pixel, against the FP64 oracle at the FP32 result's rounding."""
+    pg = circular(1, 150, 150, 0.5, nu, 49, theta0=theta)
+    for sh in _end_on(60, theta, axis).reshape(-1, 1):
+        got, _ = _gpu_project(sh, pg)
+        want = O.project_forbild(pg.to_proj_spec_array(), sh, mode=0)
+        assert want[0, nu // 2, 24] > 0.7 * 39.0
+        assert np.abs(got - want).max() <= 2e-6 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+def test_gpu_solids_beside_the_source() -> None:
+    """Solids around the source whose centre lies beside it, in front by little more than the records' rounding, project
+    to billions of pixels: the forms about that centre have no bits left at the detector's, where the general solver has
+    to run."""
+    rng = np.random.default_rng(32)
+    theta = 0.3
+    pg = circular(1, 150, 150, 0.5, 65, 49, theta0=theta)
+    sp = pg.to_proj_spec_array()[0]
+    sh = np.zeros(4000, S.forbild_shape)
+    sh["type"], sh["rho"], sh["r"] = 13, 0.4, rng.uniform(25, 60, len(sh))
+    b, e = rng.uniform(-15, 15, len(sh)), 10.0 ** rng.uniform(-9, -5, len(sh))
+    sh["x"], sh["y"] = (150 - e) * np.cos(theta) - b * np.sin(theta), (150 - e) * np.sin(theta) + b * np.cos(theta)
+    sh["z"] = rng.uniform(-5, 5, len(sh))
+    f = lambda v: np.array([v["x"], v["y"], v["z"]], np.float64)  # noqa: E731
+    n, s = np.cross(f(sp["det_u"]), f(sp["det_v"])), f(sp["source_pos"])
+    ahead = (np.stack([sh["x"], sh["y"], sh["z"]], 1).astype(np.float64) - s) @ n * np.sign((f(sp["det_pos"]) - s) @ n)
+    ahead[ahead <= 0] = np.inf
+    for k in np.argsort(ahead)[:40]:
+        got, _ = _gpu_project(sh[k : k + 1], pg)
+        want = O.project_forbild(pg.to_proj_spec_array(), sh[k : k + 1], mode=0)
+        assert want.min() > 0
+        assert np.abs(got - want).max() <= 2e-6 * want.max()
