@@ -37,32 +37,42 @@ static_assert(sizeof(aprict_forbild_shape) == 156, "FORBILD_Shape is 156 bytes i
 namespace {
 
 constexpr int kThreads = 256;
-// Shapes per shared-memory chunk (one chunk, one barrier round): as many records
-// as five resident CTAs' shared memory holds.
-constexpr int kChunk = 112;
+// Shapes per shared-memory chunk (one chunk, one barrier round): as many records of
+// 352 bytes as five resident CTAs' shared memory holds. A phantom of one chunk keeps
+// it between the sub-rays of a tile: 128 shapes with 3 x 3 sub-rays, 10 views x 512^2,
+// 1.96 ms in one chunk, 2.32 in two (records of 392 bytes, 112 a chunk).
+constexpr int kChunk = 128;
 constexpr int kMaxU = 16;   // disjoint covered intervals tracked per ray
 constexpr int64_t kScratchBytes = 256ll << 20;  // largest per-(view, shape) scratch
 
 struct QView {
     double o[3], d0[3], du[3], dv[3];  // local(t) = o + t (d0 + du fu + dv fv)
-    double cq;                         // canonical constant (see kind)
     double g0[3], gd0[3], gdu[3], gdv[3];
-    double h, alpha, beta;
-    double rho;
-    int kind, n_clip;
+    double h;
     // Ellipsoids and cylinders (fast = 1): with a = fu - uc, b = fv - vc the pixel's
     // offset from the projected centre, the ray's quadratic A t^2 + 2 B t + C has
     //   A = |d|^2, B = o.d and B^2 - A C = A - |o x d|^2
     // (Lagrange's identity; the cylinder's in its cross-section), each a
     // polynomial in (a, b): A and disc as c0 + ca a + cb b + caa a^2 + cab a b +
     // cbb b^2, B linear. At the centre o x d = 0, so disc loses nothing to the
-    // cancellation of B^2 and A C.
-    double uc, vc, A[6], B[3], disc[6];
+    // cancellation of B^2 and A C, and its constant is A's.
+    union {
+        struct {
+            double alpha, beta;  // cones
+        };
+        struct {
+            double uc, vc;  // ellipsoids, cylinders
+        };
+    };
+    double A[6], B[3], disc[5];
     double a_min;     // below it (a ray along a cylinder's axis, a centre beside the source) the general solver runs
     double disc_min;  // (negative) what a discriminant of 0 may come out as: below it the ray misses
-    int fast;
-    int between;  // every point of the solid lies strictly between the source and the detector: 0 < t < 1
+    float rho;
+    uint8_t kind, n_clip;
+    uint8_t fast;
+    uint8_t between;  // every point of the solid lies strictly between the source and the detector: 0 < t < 1
 };
+static_assert(sizeof(QView) == 352, "five CTAs per SM hold kChunk records");
 
 // ------------------------------------------------------------------ host
 void nrm3(const double a[3], double o[3]) {
@@ -378,12 +388,12 @@ __device__ void make_forms(const ViewGeom &g, const aprict_quadric &q, QView &o)
     o.B[0] = dot(o.o, c, n);
     o.B[1] = dot(o.o, o.du, n);
     o.B[2] = dot(o.o, o.dv, n);
-    o.disc[0] = o.A[0] - dot(w0, w0, 3);
-    o.disc[1] = o.A[1] - 2.0 * dot(w0, wu, 3);
-    o.disc[2] = o.A[2] - 2.0 * dot(w0, wv, 3);
-    o.disc[3] = o.A[3] - dot(wu, wu, 3);
-    o.disc[4] = o.A[4] - 2.0 * dot(wu, wv, 3);
-    o.disc[5] = o.A[5] - dot(wv, wv, 3);
+    // (w0 is the rounding of a zero: |w0|^2 is far below A[0]'s last place)
+    o.disc[0] = o.A[1] - 2.0 * dot(w0, wu, 3);
+    o.disc[1] = o.A[2] - 2.0 * dot(w0, wv, 3);
+    o.disc[2] = o.A[3] - dot(wu, wu, 3);
+    o.disc[3] = o.A[4] - 2.0 * dot(wu, wv, 3);
+    o.disc[4] = o.A[5] - dot(wv, wv, 3);
     // A's terms cancel towards a cylinder's axis, and for a centre beside the source, whose
     // direction is far longer than a pixel's: 1e-6 of their size is still good to 1e-10
     const double size = dot(o.d0, o.d0, n);
@@ -419,18 +429,12 @@ __device__ void make_qview(const ViewGeom &g, const aprict_quadric &q, QView &o)
     mul(g.D0, o.d0);
     mul(g.U, o.du);
     mul(g.V, o.dv);
-    o.kind = q.kind;
-    o.n_clip = q.n_clip & 0xFF;
-    o.rho = q.rho;
+    o.kind = (uint8_t)q.kind;
+    o.n_clip = (uint8_t)(q.n_clip & 0xFF);
+    o.rho = (float)q.rho;  // (a float in the shape)
     o.h = q.h;
     o.alpha = q.alpha;
     o.beta = q.beta;
-    if (q.kind == 1)
-        o.cq = o.o[0] * o.o[0] + o.o[1] * o.o[1] + o.o[2] * o.o[2] - 1.0;
-    else if (q.kind == 2)
-        o.cq = o.o[0] * o.o[0] + o.o[1] * o.o[1] - 1.0;
-    else
-        o.cq = 0.0;
     make_forms(g, q, o);
     for (int k = 0; k < 3; ++k) {
         if (k < (q.n_clip & 0xFF)) {
@@ -470,8 +474,9 @@ __device__ __forceinline__ void slab(double o, double d, double h, double &lo, d
     hi = fmin(hi, fmax(t0, t1));
 }
 
-__device__ __forceinline__ double form6(const double (&c)[6], double a, double b) {
-    return fma(b, fma(b, c[5], c[2]), fma(a, fma(a, c[3], fma(b, c[4], c[1])), c[0]));
+// c0 + c[0] a + c[1] b + c[2] a^2 + c[3] a b + c[4] b^2
+__device__ __forceinline__ double form2(double c0, const double *c, double a, double b) {
+    return fma(b, fma(b, c[4], c[1]), fma(a, fma(a, c[2], fma(b, c[3], c[0])), c0));
 }
 
 // Parametric interval of the ray with the clipped shape, within [0, 1]: the
@@ -501,11 +506,11 @@ __device__ __noinline__ bool ray_interval_general(const QView &q, double fu, dou
     if (q.kind == 1) {
         A = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         B = o[0] * d[0] + o[1] * d[1] + o[2] * d[2];
-        C = q.cq;
+        C = o[0] * o[0] + o[1] * o[1] + o[2] * o[2] - 1.0;
     } else if (q.kind == 2) {
         A = d[0] * d[0] + d[1] * d[1];
         B = o[0] * d[0] + o[1] * d[1];
-        C = q.cq;
+        C = o[0] * o[0] + o[1] * o[1] - 1.0;
     } else {
         const double ra = q.alpha + q.beta * o[2], rb = q.beta * d[2];
         A = d[0] * d[0] + d[1] * d[1] - rb * rb;
@@ -569,9 +574,9 @@ __device__ __noinline__ bool ray_interval_general(const QView &q, double fu, dou
 __device__ __forceinline__ bool ray_interval(const QView &q, double fu, double fv, double &lo, double &hi) {
     if (!q.fast) return ray_interval_general(q, fu, fv, lo, hi);
     const double a = fu - q.uc, b = fv - q.vc;
-    const double disc = form6(q.disc, a, b);
+    const double disc = form2(q.A[0], q.disc, a, b);
     if (!(disc > q.disc_min)) return false;
-    const double A = form6(q.A, a, b);
+    const double A = form2(q.A[0], q.A + 1, a, b);
     if (!(A > q.a_min)) return ray_interval_general(q, fu, fv, lo, hi);
     // a chord below 1e-10 of the solid's size is under the discriminant's own rounding
     if (!(disc > 1e-20 * A)) return false;
@@ -651,8 +656,7 @@ TileMap make_tiles(uint32_t nu, uint32_t nv) {
 // k_forbild_prep (85.3 ms with them in the same kernel as the in-tile
 // derivation, 70.9 ms in a variant without it: fewer spills; 81.6 ms at 6
 // CTAs per SM; 65.2 ms with one reciprocal for both quadric roots). The records
-// of the polynomial forms (ray_interval) are larger, so that a chunk of 112
-// shapes is what five CTAs' shared memory holds; all threads copy the kept ones.
+// of the polynomial forms (ray_interval) are copied by all threads.
 template <int MODE, bool PRE>
 __global__ void __launch_bounds__(kThreads, 5) k_project_forbild(const aprict_proj_spec *__restrict__ specs,
                                                                uint32_t n_views, uint32_t nu, uint32_t nv,
@@ -763,12 +767,12 @@ __global__ void __launch_bounds__(kThreads, 5) k_project_forbild(const aprict_pr
                         double lo, hi;
                         if (!ray_interval(q, fu, fv, lo, hi)) continue;
                         if (MODE != 0) {
-                            val += q.rho * (hi - lo);
+                            val += (double)q.rho * (hi - lo);
                             continue;
                         }
                         double covered = 0.0;
                         for (int i = 0; i < m; ++i) covered += fmax(0.0, fmin(hi, uR[i]) - fmax(lo, uL[i]));
-                        val += q.rho * ((hi - lo) - covered);
+                        val += (double)q.rho * ((hi - lo) - covered);
                         double a = lo, b = hi;
                         int wpos = 0;
                         for (int i = 0; i < m; ++i) {

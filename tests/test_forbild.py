@@ -136,7 +136,7 @@ def test_gpu_matches_oracle_all_types(mode_kw: dict, mode: int) -> None:
 
 @pytest.mark.gpu
 def test_gpu_supersampling_multiply_and_chunks() -> None:
-    """More shapes than one shared-memory chunk (96), ssu/ssv > 1, mba != 1."""
+    """More shapes than one shared-memory chunk (128), ssu/ssv > 1, mba != 1."""
     rng = np.random.default_rng(12)
     shapes = random_shapes_all_types(rng, 200, radius=60)
     pg = circular(4, 150, 150, 0.5, 48, 40)
@@ -284,3 +284,14 @@ def test_gpu_solids_beside_the_source() -> None:
         want = O.project_forbild(pg.to_proj_spec_array(), sh[k : k + 1], mode=0)
         assert want.min() > 0
         assert np.abs(got - want).max() <= 2e-6 * want.max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [127, 128, 129])
+def test_gpu_around_one_chunk(n: int) -> None:
+    """Phantoms of one chunk (kept between the sub-rays of a tile) and of one shape more."""
+    shapes = random_shapes_all_types(np.random.default_rng(n), n, radius=60)
+    pg = circular(2, 150, 150, 0.5, 48, 40)
+    got, _ = _gpu_project(shapes, pg, ssu=2, ssv=2)
+    want = O.project_forbild(pg.to_proj_spec_array(), shapes, mode=0, ssu=2, ssv=2)
+    assert rel_l2(got, want) <= 1e-5
