@@ -750,13 +750,16 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
 // taken by four-point Lagrange interpolation for each (radius, angle): 4096
 // height sums instead of n_r num_ang of them (396 x 6000: 2.4 million).
 // Interpolation error, relative to F, node spacing h: (h / ell)^4 from the
-// smooth part, below 4e-9 where ell >= 128 h; and from the window, whose
-// second derivative jumps at its two edges by up to 6 gamma^2 (ds/d ell)^2,
-// |ds/d ell| <= 0.4 / ell: at a given ell only the samples within one node of
-// an edge feel it, a share of about h, hence at most 0.12 gamma^2 h^3 / ell^2,
-// 2e-8 for gamma <= 200 at h = 1.5e-4. Both lie below the FP32 rounding of the
-// samples. (radius, angle) pairs with ell < 128 h, and calls with a steeper
-// window (kMaxGamma) or without scratch for the table sum their heights directly.
+// smooth part, below 4e-9 where ell >= 128 h; and from the window, whose second
+// derivative jumps at its two edges. A sample whose edge lies within a node of ell
+// is off by a share of gamma^2 (h / ell)^2, and of the N = ell (num_z - 1) /
+// (1 + r_max) samples in the window there are about N h / ell of them, at least
+// one now and then:
+//   error <= 0.06 gamma^2 (h / ell)^2 max(h / ell, 1 / N)
+// (the rule in FP64 over window angles 0.1 .. 1, r_max 0.3 .. 1.1, gamma 5 .. 193, 100 ..
+// 6000 heights: 0.045 at most). Where that exceeds kTol, a third of the samples'
+// FP32 rounding, and below 128 h, the heights are summed directly, as in calls
+// without scratch for the table.
 // 396 radii x 6000 x 6000 samples, the whole call: 7.0 -> 0.55 ms (most of it host
 // work; sums equal to 1e-8).
 // sin^2 theta grows with z, so a height sum stops at the first height past the
@@ -765,7 +768,7 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
 // radius an FP64 block sum over angles and one atomic add.
 constexpr int kNodes = 4096;        // interpolation nodes of the height sum
 constexpr int kDirectBelow = 128;   // node spacings below which ell is summed directly
-constexpr float kMaxGamma = 200.f;  // steepest window (1 / sine width of its band) that is interpolated
+constexpr float kTol = 2e-8f;       // largest relative error of an interpolated height sum
 constexpr int kZRun = 64;  // heights per FP32 partial sum
 
 // sum over heights iz = 0 .. num_z - 1 (iz = 0 with weight 1/2) of
@@ -850,12 +853,21 @@ __device__ __forceinline__ void ell_nodes(float r_max, float &lo, float &h) {
     lo -= h;
 }
 
+// The least ell that is interpolated (see above; infinite for a steep window).
+__device__ __forceinline__ float ell_direct(float r_max, float lo, float h, int num_z, const SoftWin &v) {
+    if (!(h > 0.f)) return INFINITY;
+    const float gh = v.gamma * h;
+    const float edge = cbrtf(0.06f / kTol * gh * gh * fmaxf(h, (1.f + r_max) / (float)(num_z - 1)));
+    return edge >= 0.f ? fmaxf(edge, fmaxf((float)kDirectBelow * h, lo + h)) : INFINITY;
+}
+
 __global__ void __launch_bounds__(kGThreads) k_gbc_height_table(const float *r_on_R, int nr, double *table, int num_z, SoftWin v,
                                                                 float tan_v) {
     const int lane = threadIdx.x & 31, node = (blockIdx.x * kGThreads + threadIdx.x) >> 5;
     if (node >= kNodes) return;
     float lo, h;
     ell_nodes(r_on_R[nr - 1], lo, h);
+    if (fmaf((float)(node + 3), h, lo) < ell_direct(r_on_R[nr - 1], lo, h, num_z, v)) return;  // never read
     const float dz = tan_v * (1.f + r_on_R[nr - 1]) / (float)(num_z - 1);
     double s = height_sum_lane(fmaxf(0.f, fmaf((float)node, h, lo)), num_z, dz, v, lane);
 #pragma unroll
@@ -883,7 +895,7 @@ __global__ void __launch_bounds__(kGThreads) k_gbc_weight_integ(const float *r_o
     const float dz = maxz / (float)(num_z - 1);
     float lo, h;
     ell_nodes(r_on_R[nr - 1], lo, h);
-    const float direct = table && h > 0.f ? fmaxf((float)kDirectBelow * h, lo + h) : INFINITY;
+    const float direct = table ? ell_direct(r_on_R[nr - 1], lo, h, num_z, S.v) : INFINITY;
     const double mult = (double)((4.f * maxz * 3.1415926535898f) / ((float)num_z * (float)num_ang));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int r = blockIdx.y; r < nr; r += gridDim.y) {
@@ -1141,8 +1153,7 @@ extern "C" int aprict_b200_gbc_weight_integral_scratch(const float *r_on_R_dev, 
     if ((reinterpret_cast<uintptr_t>(scratch_dev) & 7u) != 0)
         return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "gbc_weight_integral: scratch not 8-byte aligned");
     double *table = static_cast<double *>(scratch_dev);
-    if (table != nullptr && std::fabs(S.v.gamma) <= kMaxGamma &&
-        aprict_b200_gbc_weight_integral_scratch_bytes(n_r, num_ang) > 0) {
+    if (table != nullptr && aprict_b200_gbc_weight_integral_scratch_bytes(n_r, num_ang) > 0) {
         k_gbc_height_table<<<kNodes * 32 / kGThreads, kGThreads, 0, st>>>(r_on_R_dev, n_r, table, num_z, S.v, tan_v);
         // a CTA per radius where the radii alone fill the GPU
         const int per_r = n_r >= 296 ? 1 : (num_ang + kGThreads - 1) / kGThreads;

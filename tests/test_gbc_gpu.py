@@ -110,12 +110,11 @@ def test_weight_integral_edges(r: np.ndarray, nz: int, na: int, soft: tuple) -> 
     (np.linspace(0.3, 0.0, 40), 200, 700, SOFT),                       # radii out of order: outside the nodes
     (np.zeros(1), 300, 20000, SOFT),                                   # no range of ell
     (np.linspace(0.0, 0.3, 40), 500, 700, (0.22, 0.002, 0.45, 0.05)),  # a steep window: summed directly
-    (np.linspace(0.0, 0.3, 40), 500, 700, (0.22, 0.0065, 0.45, 0.05)),  # just below the steepest interpolated
+    (np.linspace(0.0, 0.3, 40), 500, 700, (0.22, 0.0065, 0.45, 0.05)),  # steep: the smaller ell summed directly
     (np.linspace(0.0, 0.3, 40), 300, 700, (2.0, 0.1, 1.7, 0.3)),
 ])
 def test_weight_integral_table(r: np.ndarray, nz: int, na: int, soft: tuple) -> None:
-    """Calls large enough for the table of inner sums. The interpolation's error stays below 1e-7 (derived
-    beside the kernel); the gate is the direct sums'."""
+    """Calls large enough for the table of inner sums, against the oracle; the gate is the direct sums'."""
     cfg = fp.ConfigBackproject(fast_approx=True, backproj_weighting_preset=7, Z_on_val_factor_val=60.0,
                                approx_mode_direct_raycast=True, soft_vartheta_v=soft[0],
                                soft_vartheta_v_softspan=soft[1], soft_vartheta_h=soft[2],
@@ -123,6 +122,34 @@ def test_weight_integral_table(r: np.ndarray, nz: int, na: int, soft: tuple) -> 
     got = gbc.backproj_gbc_weight_integ_GPU(r, cfg, nz, na)
     want = G.weight_integral(r.astype(np.float32), soft, nz, na)
     np.testing.assert_allclose(got, want, rtol=1e-5, atol=1e-6 * float(np.abs(want).max()))
+
+
+@pytest.mark.parametrize(("r_max", "nz", "gamma"), [(0.95, 500, 193), (0.95, 100, 193), (0.95, 6000, 193), (0.95, 500, 20),
+                                                    (0.6, 500, 193), (0.3, 100, 193), (0.3, 6000, 20), (1.1, 300, 60)])
+def test_weight_integral_table_against_direct_sums(r_max: float, nz: int, gamma: float) -> None:
+    """Few angles, which average no interpolation error away: the call with the table against the call without.
+    Interpolated inner sums carry at most 2e-8; a direct or a node's sum has FP32 samples, whose reciprocal root's cube
+    is good to 3 x 2 units of 2^-24 and its four products to one each: 10 x 6e-8."""
+    from aprict_b200 import _lib
+
+    a = 0.5
+    soft = (a, float(a - np.arcsin(np.sin(a) - 1 / gamma)), 0.45, 0.05)
+    cfg = fp.ConfigBackproject(fast_approx=True, backproj_weighting_preset=7, Z_on_val_factor_val=60.0,
+                               approx_mode_direct_raycast=True, soft_vartheta_v=soft[0], soft_vartheta_v_softspan=soft[1],
+                               soft_vartheta_h=soft[2], soft_vartheta_h_softspan=soft[3]).contents
+    r = torch.linspace(0, r_max, 2100, dtype=torch.float32, device="cuda")
+    lib, na = _lib.lib(), 8
+    nbytes = lib.aprict_b200_gbc_weight_integral_scratch_bytes(len(r), na)
+    assert nbytes > 0
+    out = []
+    for scratch in (torch.empty(nbytes, dtype=torch.uint8, device="cuda"), None):
+        o = torch.zeros(len(r), dtype=torch.float64, device="cuda")
+        _lib.check(lib.aprict_b200_gbc_weight_integral_scratch(
+            r.data_ptr(), len(r), o.data_ptr(), nz, na, _lib.ptr(cfg), None if scratch is None else scratch.data_ptr(),
+            torch.cuda.current_stream().cuda_stream), "gbc_weight_integral")
+        out.append(o.cpu().numpy())
+    assert out[1].min() > 0
+    assert np.abs(out[0] / out[1] - 1).max() <= 6e-7
 
 
 @pytest.mark.parametrize("nz", [9, 33, 65, 130, 257])
