@@ -655,6 +655,11 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
                             const f32x2 x = pk(__saturatef(fmaf(G.soft.v.gamma, fabsf(za) * ia, -G.soft.v.chi)),
                                                __saturatef(fmaf(G.soft.v.gamma, fabsf(zb) * ib, -G.soft.v.chi)));
                             w = mul2(w, mul2(mul2(x, x), fma2(x, pk(-2.f, -2.f), pk(3.f, 3.f))));
+                            // past the window nothing is sampled: 0 times an infinite pixel is no 0
+                            float wa, wb, sa, sb;
+                            upk(w, wa, wb);
+                            upk(pv, sa, sb);
+                            pv = pk(wa == 0.f ? 0.f : sa, wb == 0.f ? 0.f : sb);
                         }
                         accw2[k] = add2(accw2[k], w);
                         acc2[k] = fma2(pv, w, acc2[k]);

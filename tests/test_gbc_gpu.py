@@ -173,6 +173,30 @@ def test_columns_match_oracle(nz: int, linear: bool, soft: tuple) -> None:
     assert rel_l2(ws.as_numpy(), want_w) <= 1e-5
 
 
+@pytest.mark.parametrize("linear", [False, True])
+def test_non_finite_pixels_outside_the_window(linear: bool) -> None:
+    """Infinite and NaN pixels reach the voxels that sample them inside the vertical window and no others: blocks
+    of a column across the window's end weigh the pixels past it with 0."""
+    pg = _scan(m=12, h=0.0, nu=31, nv=160)
+    projs = np.random.default_rng(9).random((12, 31, 160)).astype(np.float32)
+    projs[3, 14, 30:60], projs[7, 18, 100:150] = np.inf, np.nan
+    cfg = fp.ConfigBackproject(fast_approx=True, backproj_weighting_preset=7, Z_on_val_factor_val=60.0, soft_vartheta_v=0.35,
+                               soft_vartheta_v_softspan=0.1, soft_vartheta_h=0.45, soft_vartheta_h_softspan=0.05,
+                               approx_mode_direct_raycast=True, approx_mode_bilinear_interpolate=linear)
+    out = []
+    for views in (1, 2):
+        v, ws = Volume.zeros((20, 18, 120), voxwid=0.83), Volume.zeros((20, 18, 120), voxwid=0.83)
+        ps = fp.ProjectionSet(pg, data=projs)
+        ps._backproject_promise = lambda needs_z, views=views: views  # noqa: SLF001
+        fp.backproject(cfg, v, ps, secondary_volume=ws, block=True)
+        assert np.isfinite(ws.as_numpy()).all()
+        out.append(v.as_numpy())
+    bad = ~np.isfinite(out[1])
+    assert bad.any() and not bad.all()
+    np.testing.assert_array_equal(~np.isfinite(out[0]), bad)
+    assert rel_l2(out[0][~bad], out[1][~bad]) <= (1e-5 if linear else 1e-6)
+
+
 @pytest.mark.parametrize(("shape", "nu", "nv"), [((20, 22, 33), 31, 40), ((21, 19, 64), 30, 41)])
 def test_exact_ties_fall_as_in_the_general_kernel(shape: tuple, nu: int, nv: int) -> None:
     """As the columns' test of the same name: mid plane or axis between two pixels in every view of a circular scan."""
