@@ -18,12 +18,17 @@
 // fma; the arithmetic runs on pairs of voxels (fma.rn.f32x2).
 //
 // Row choice: A and S come from FP64, so the FP32 row coordinate is off by at
-// most u (2 |A| + 2 |n S| + |f|), u = 2^-24, some 5e-5 pixel on a 384-row
-// detector (ten times less than with forms rounded before the division). A
-// row whose fraction comes that close to 1/2 is decided again in FP64; such a
-// voxel-view occurs in about 2 % of the warp's views, so it is settled at
-// once, the difference to the pixel already gathered going to the voxel's
-// compensated total.
+// most u (|A| + 3 |n S| + 3 |f|), u = 2^-24 (A, S and three sums rounded, of which
+// the first two may exceed f by n S): some 5e-5 pixel on a 384-row detector (ten
+// times less than with forms rounded before the division). The bound depends on the
+// volume's height, not on XB, so that a column settles the same rows in a batch. A
+// row whose fraction comes that close to 1/2 is decided again in FP64. Such a
+// voxel-view occurs in about 2 % of a warp's views, and in every view where a grid
+// of odd height has its mid plane on the edge between two rows: it is set to 0,
+// queued per warp and settled with up to 31 others, one per lane, its product going
+// to the voxel's compensated total. 255^3 x 120 views, mid plane and axis on edges:
+// 2.15 ms (settled at once, by a call in the view loop: 3.83 ms; 256^3 x 180 views,
+// no edges: 1.69 and 1.82 ms).
 //
 // Bound: gather latency and issue (on 256^3 x 360 views x 384^2 nearest: 12.5
 // warp instructions per 32 voxel-views against 21 of the brick kernel's z-lane
@@ -34,11 +39,9 @@
 // registers, no spills: 3.6 ms.
 //
 // Columns cut by the detector's edges (helical scans; 256^3 x 180 views, one
-// turn): nearest 7.2 -> 3.8 ms, direct raycast 6.3 -> 2.8 ms. Their blocks are
+// turn): nearest 6.4 -> 2.5 ms, direct raycast 7.7 -> 2.6 ms. Their blocks are
 // gathered under a predicate (a branch around the gather: twice the time), blocks
-// inside four at a time, and their close rows settled together with the others'
-// (a call in each block, around which the column's registers spill: 5.2 and 3.6
-// ms, and 1.62 instead of 1.57 ms on the circular scan, which has no such column).
+// inside four at a time.
 #pragma once
 
 #include "ab_bpbrick.cuh"
@@ -73,6 +76,14 @@ struct ColSmem {
     ColRec rec[kColWarps][32];
     float ksum[kColWarps][32 * XB];   // compensated totals over the view chunks
     float kcomp[kColWarps][32 * XB];
+    double pos[kColWarps][4];         // the warp's column: x, y relative to the volume centre, height of voxel 0 in voxels
+    struct {                          // what col_settle takes from the call's parameters
+        double vwd;
+        float sep, inv_sep;
+        int nv;
+        uint32_t sv4;
+    } par;
+    uint16_t q[kColWarps][64];        // close voxel-views: view of the group | block << 5 | lane << 8
 };
 
 // ab_derive_bpview's FP64 forms for an upright view with the vanishing terms
@@ -129,6 +140,49 @@ static __device__ __noinline__ float col_exact_row(const ab_bpview_d &d, double 
                : 0.f;
 }
 
+// The FP32 row coordinate of lane `lane`'s voxel in block k, as the pairs of blocks form it.
+__device__ __forceinline__ float col_row(const float4 &a, int lane, int k) {
+    const float f = fmaf((float)lane, a.y, a.x), s32 = 32.f * a.y, fo = (k & 1) ? f + s32 : f;
+    return k < 2 ? fo : fmaf((float)(k & ~1), s32, fo);
+}
+
+// Settles the first c <= 32 close voxel-views of a warp's queue, one per lane, and
+// adds their products to the totals in queue order. A call: rare.
+template <int XB>
+static __device__ __noinline__ void col_settle(ColSmem<XB> &sm, int g0, int c) {
+    __syncwarp();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = sm.par.nv;
+    const float sep = sm.par.sep;
+    const unsigned e = lane < c ? sm.q[warp][lane] : 0u;
+    float pe = 0.f;
+    if (lane < c) {
+        const int j = e & 31, k = (e >> 5) & 7, l = e >> 8;
+        const ColRec &rc = sm.rec[warp][j];
+        const float4 ra = rc.a;
+        const float fc = fminf(fmaxf(col_row(ra, l, k), -2097152.f), 2097152.f);
+        const int crow = nv >> 1;
+        const double *pos = sm.pos[warp];
+        pe = col_exact_row(sm.view[g0 + j].d, pos[0], pos[1], (pos[2] + (double)(l + 32 * k)) * sm.par.vwd, fc, crow,
+                           nv, ((uint64_t)rc.b.y << 32) | rc.b.x, sm.par.sv4);
+        const float rv = fabsf(fc - (0.5f * ((float)nv - 1.f) - (float)crow)), halfv = 0.5f * (float)nv;
+        if (sep > 0.f && rv > halfv * ((1.f - sep) * (1.f - 1e-5f)) && pe != 0.f)
+            pe *= ab_edge_taper_half(rv, 2.f / (float)nv, sm.par.inv_sep);
+    }
+    for (int i = 0; i < c; ++i) {  // each voxel's products in order, on the lane that owns it
+        const unsigned ei = __shfl_sync(0xffffffffu, e, i);
+        const float p = __shfl_sync(0xffffffffu, pe, i);
+        if (lane == (int)(ei >> 8)) {
+            const int o = lane + 32 * (int)((ei >> 5) & 7);
+            const float sk = sm.ksum[warp][o];
+            const float y = fmaf(p, sm.rec[warp][ei & 31].a.z, -sm.kcomp[warp][o]);
+            const float tk = sk + y;
+            sm.kcomp[warp][o] = (tk - sk) - y;
+            sm.ksum[warp][o] = tk;
+        }
+    }
+    __syncwarp();
+}
+
 // Backprojects scan P, all of whose views are upright, into the columns of work unit
 // `brick` (in P.col's order). Every thread of the CTA calls it.
 // BILIN (v stride 1): two pixel columns and the weight between them in the
@@ -174,13 +228,24 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
     const f32x2 magic = pk(kMagic, kMagic), nmagic = pk(-kMagic, -kMagic), minus1 = pk(-1.f, -1.f);
     const f32x2 one = pk(1.f, 1.f), mhalf = pk(-0.5f, -0.5f);
 
+    if (threadIdx.x == 0) {
+        sm.par.vwd = P.vwd;
+        sm.par.sep = P.sep;
+        sm.par.inv_sep = P.inv_sep;
+        sm.par.nv = (int)P.nv;
+        sm.par.sv4 = sv4;
+    }
     for (int isub = 0; isub < n_sub; ++isub) {
         const double fx = -0.5 + (0.5 + isub / (P.ssy * P.ssz)) / P.ssx;
         const double fy = -0.5 + (0.5 + (isub / P.ssz) % P.ssy) / P.ssy;
         const double fz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
         // the column's first voxel relative to the volume centre
-        const double X = (ix + 0.5 + fx - 0.5 * P.n[0]) * P.vwd, Y = (iy + 0.5 + fy - 0.5 * P.n[1]) * P.vwd;
-        const double zi0 = z0 + 0.5 + fz - 0.5 * P.n[2], Z0 = zi0 * P.vwd;
+        // (kept in shared memory: the view loop has no registers for it)
+        if (lane == 0) {
+            sm.pos[warp][0] = (ix + 0.5 + fx - 0.5 * P.n[0]) * P.vwd;
+            sm.pos[warp][1] = (iy + 0.5 + fy - 0.5 * P.n[1]) * P.vwd;
+            sm.pos[warp][2] = z0 + 0.5 + fz - 0.5 * P.n[2];
+        }
         for (uint32_t v0 = 0; v0 < P.n_views; v0 += kChunk) {
             const int cn = (int)min((uint32_t)kChunk, P.n_views - v0);
             __syncthreads();
@@ -212,6 +277,7 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
 #pragma unroll
             for (int k = 0; k < XB / 2; ++k) pvp[k] = pk(0.f, 0.f);
             float wp = 0.f;
+            int qn = 0;  // close voxel-views queued
             f32x2 acc2[XB / 2];
 #pragma unroll
             for (int k = 0; k < XB / 2; ++k) acc2[k] = pk(0.f, 0.f);
@@ -225,6 +291,7 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                     rec.b = make_uint4(0u, 0u, 0u, 0u);
                     if (t < cn && sm.view[t].ok) {
                         const ColView &cv = sm.view[t];
+                        const double X = sm.pos[warp][0], Y = sm.pos[warp][1], Z0 = sm.pos[warp][2] * P.vwd;
                         const double D = fma(cv.d.den[0], X, fma(cv.d.den[1], Y, cv.d.den[3]));
                         const double rD = 1.0 / D;
                         const double fu = fma(cv.d.nu[0], X, fma(cv.d.nu[1], Y, cv.d.nu[3])) * rD;
@@ -250,10 +317,11 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                                 }
                                 const float cu = fabsf((float)(fu - 0.5 * ((double)P.nu - 1.0)));
                                 if (P.sep > 0.f) w *= ab_edge_taper_half(cu, 2.f / (float)P.nu, P.inv_sep);
-                                // error of the FP32 row coordinate, with a margin of 1.5, and where each
-                                // block of 32 voxels projects (with that error to spare)
-                                const float eps = fmaf(1.5f * 5.9604645e-8f,
-                                                       3.f * fabsf(Af) + (3.f * 32 * XB) * fabsf(Sf) + (float)P.nv, 1e-6f);
+                                // error of the FP32 row coordinate, and where each block of 32 voxels
+                                // projects (with that error to spare)
+                                const float eps = fmaf(1.05f * 5.9604645e-8f,
+                                                       fmaf(3.f * (float)min(P.n[2] - z0, 256), fabsf(Sf), fabsf(Af)) +
+                                                           (1.5f * (float)P.nv + 3.f), 1e-6f);
                                 unsigned in = 0, across = 0;
 #pragma unroll
                                 for (int k = 0; k < XB; ++k) {
@@ -395,26 +463,41 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
                             }
                         }
                     }
-                    if (!BILIN && tie > ra.w) {  // some row of this lane is too close to call in FP32
-#pragma unroll 1
-                        for (int k = 0; k < XB; ++k) {
-                            const float fo = (k & 1) ? a + s32 : a;
-                            const float f = k < 2 ? fo : fmaf((float)(k & ~1), s32, fo);
-                            const float fc = fminf(fmaxf(f, -2097152.f), 2097152.f);
-                            const float d = __fsub_rn(fc, __fsub_rn(__fadd_rn(fc, kMagic), kMagic));
-                            if (!((in | across) >> k & 1u) || fabsf(d) <= ra.w) continue;
-                            float pe = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, fc,
-                                                     crow, (int)P.nv, col, sv4);
-                            const float rv = fabsf(fc - coff);
-                            if (P.sep > 0.f && rv > flatv && pe != 0.f) pe *= ab_edge_taper_half(rv, inv_halfv, P.inv_sep);
+                    if (!BILIN && __any_sync(0xffffffffu, tie > ra.w)) {  // rows too close to call in FP32
+                        unsigned close = 0;
 #pragma unroll
-                            for (int m = 0; m < XB / 2; ++m) {  // registers: the index has to be constant
-                                float q0, q1;
-                                upk(pvp[m], q0, q1);
-                                pvp[m] = pk(k == 2 * m ? pe : q0, k == 2 * m + 1 ? pe : q1);
+                        for (int m = 0; m < XB / 2; ++m) {
+                            const f32x2 f = m == 0 ? f0 : fma2(pk(2.f * m, 2.f * m), s2, f0);
+                            const f32x2 d = fma2(add2(add2(f, magic), nmagic), minus1, f);
+                            float da, db, qa, qb;
+                            upk(d, da, db);
+                            upk(pvp[m], qa, qb);
+                            const bool ca = fabsf(da) > ra.w, cb = fabsf(db) > ra.w;
+                            pvp[m] = pk(ca ? 0.f : qa, cb ? 0.f : qb);
+                            close |= (ca ? 1u << (2 * m) : 0u) | (cb ? 2u << (2 * m) : 0u);
+                        }
+                        // on the detector and in the volume
+                        close &= (in | across) & ((1u << min(XB, max(0, (P.n[2] - z0 - lane + 31) >> 5))) - 1u);
+                        while (const unsigned lanes = __ballot_sync(0xffffffffu, close != 0u)) {
+                            if (close) {
+                                const int k = __ffs(close) - 1;
+                                sm.q[warp][qn + __popc(lanes & ((1u << lane) - 1u))] = (uint16_t)(j | k << 5 | lane << 8);
+                                close &= close - 1u;
+                            }
+                            qn += __popc(lanes);
+                            if (qn >= 32) {
+                                col_settle(sm, g0, 32);
+                                qn -= 32;
+                                const uint16_t rest = lane < qn ? sm.q[warp][32 + lane] : (uint16_t)0;
+                                __syncwarp();
+                                if (lane < qn) sm.q[warp][lane] = rest;
                             }
                         }
                     }
+                }
+                if (!BILIN && qn != 0) {
+                    col_settle(sm, g0, qn);
+                    qn = 0;
                 }
             }
             // the chunk's partial sums into the compensated totals

@@ -171,3 +171,26 @@ def test_columns_cut_by_the_detector(mode: str, pitch: float) -> None:
         got = _run(mode, pg, data, shape)
         assert rel_l2(got, want) <= 1e-5
         assert rel_l2(_run(mode, pg, data, shape, views=2), got) <= (1e-5 if "bilinear" in mode else 1e-6)
+
+
+@pytest.mark.parametrize("mode", ["nearest-taper", "raycast"])
+@pytest.mark.parametrize("nz", [33, 65, 97, 161, 257])
+def test_many_close_rows(mode: str, nz: int) -> None:
+    """More close rows in a group of views than a warp's queue of 32 holds, the rest of a queue at a group's end, and
+    the same voxel many times: at magnification 1 on detector rows of half and of a whole voxel nearly all of a
+    column's rows are edges between pixels (offset by 2e-6 pixel so that FP64 and the oracle agree on them), or its
+    mid plane is in every view. Bit for bit alike in a batch, whose columns take other block counts."""
+    for pix, off in ((1.0, 0.5 - 2e-6), (0.5, 0.25 - 1e-6)):
+        n, nv = 6, int(nz / pix) + 9
+        t = 0.3 + 2 * np.pi * np.arange(70) / 70
+        c, s = np.cos(t), np.sin(t)
+        L = 4e6  # a source so far that the magnification is 1 to 1e-6 over the volume
+        pg = fp.ProjGeom(source_pos=np.stack([L * c, L * s, 0 * t + off], 1), det_pos=np.stack([-40 * c, -40 * s, 0 * t + off], 1),
+                         det_uvec=0.913 * np.stack([-s, c, 0 * t], 1), det_vvec=np.tile([0.0, 0.0, -pix], (70, 1)), nu=15, nv=nv)
+        data, shape = _data(pg, nz), (n, n, nz)
+        got, bricks = _run(mode, pg, data, shape), _run(mode, pg, data, shape, views=2)
+        assert np.linalg.norm(bricks) > 0
+        assert rel_l2(got, bricks) <= 1e-6
+        v = Volume.zeros(shape, voxwid=1.0)
+        ScanBatch([v], [fp.ProjectionSet(pg, data=data)]).backproject(fp.ConfigBackproject(**MODES[mode]), block=True)
+        np.testing.assert_array_equal(v.as_numpy(), got)
