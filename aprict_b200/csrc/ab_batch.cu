@@ -27,7 +27,7 @@
 
 namespace {
 
-constexpr uint32_t kPlanMagic = 0x41424233u;  // "ABB3"
+constexpr uint32_t kPlanMagic = 0x41424234u;  // "ABB4"
 constexpr int kGroup = 96;                    // scans per launch (kernel-parameter space)
 
 // Plan layout (host image; the caller's device copy is used only for the
@@ -163,20 +163,19 @@ __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::bp_min_blocks(XB, EXAC
     retire(A.g);
 }
 
-// Batches of the fast modes on volumes of more than one layer run
-// as two launches over the same units: the scans whose views are all upright
-// take the z columns (8 voxels per thread whatever the scan's height; blocks
-// above a volume are skipped), the others the bricks. Each launch passes over
-// the other's units, after reading their views' records where the plan's maker
-// promised nothing; a batch of scans promised general is one launch.
-template <bool RAYCAST, bool BILIN>
+// Batches with scans that may take the z columns run as two launches over the same
+// units (one where every scan is promised to): scans whose views are all upright
+// take the columns (voxels per thread for the tallest of them; blocks above a volume
+// are skipped), the others the bricks. Each launch passes over the other's units,
+// after reading their views' records where the plan's maker promised nothing.
+template <bool RAYCAST, bool BILIN, int XB>
 __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::kColBlocks)
     k_batch_columns(const __grid_constant__ BatchArgs<ab_bp::BPParams> A) {
-    __shared__ ab_bp::ColSmem<8> sm;
+    __shared__ ab_bp::ColSmem<XB> sm;
     uint32_t unit;
     int s;
     while (next_unit(A, unit, s)) {
-        if (ab_bp::all_upright(A.scans[s])) ab_bp::bp_columns<RAYCAST, BILIN, 8>(A.scans[s], unit, sm);
+        if (ab_bp::all_upright(A.scans[s])) ab_bp::bp_columns<RAYCAST, BILIN, XB>(A.scans[s], unit, sm);
     }
     retire(A.g);
 }
@@ -185,8 +184,9 @@ __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::kColBlocks)
 // mode 0 fast nearest, 1 fast bilinear, 2 raycast nearest, 3 raycast
 // bilinear, 4 exact; 15: fast nearest in the z-lane layout (ORD 3) with 4
 // voxels per thread, 16: the same with 8 (every scan at least 256 voxels tall).
-// kCols is added where the scans may take the z columns.
-constexpr int kCols = 32;
+// kCols times 1, 2 or 4 (the columns' XB 2, 4 or 8) is added where scans may take the
+// z columns, kNoBricks where all are promised to.
+constexpr int kCols = 32, kColsMask = 7 * kCols, kNoBricks = 256;
 int bp_variant(const aprict_backproject_config *c, const aprict_vol_desc *vd) {
     const int mode = c->exact ? 4
                               : (c->approx_mode_direct_raycast ? 2 : 0) + (c->approx_mode_linear_interpolate ? 1 : 0);
@@ -207,14 +207,23 @@ auto bp_kernel() {
 }
 
 // The z-column kernel of a variant code's mode (15 and 16 are mode 0).
+template <int XB, class F>
+int with_columns_kernel_of(int v, F &&f) {
+    switch (v < 15 ? v / 3 : 0) {
+        case 1: return f(k_batch_columns<false, true, XB>);
+        case 2: return f(k_batch_columns<true, false, XB>);
+        case 3: return f(k_batch_columns<true, true, XB>);
+        default: return f(k_batch_columns<false, false, XB>);
+    }
+}
+
 template <class F>
 int with_columns_kernel(int variant, F &&f) {
     const int v = variant & (kCols - 1);
-    switch (v < 15 ? v / 3 : 0) {
-        case 1: return f(k_batch_columns<false, true>);
-        case 2: return f(k_batch_columns<true, false>);
-        case 3: return f(k_batch_columns<true, true>);
-        default: return f(k_batch_columns<false, false>);
+    switch ((variant & kColsMask) / kCols) {
+        case 1: return with_columns_kernel_of<2>(v, f);
+        case 2: return with_columns_kernel_of<4>(v, f);
+        default: return with_columns_kernel_of<8>(v, f);
     }
 }
 
@@ -244,7 +253,7 @@ int with_bp_kernel_of(int variant, F &&f) {
 
 template <class F>
 int with_bp_kernel(int variant, F &&f) {
-    return variant & kCols ? with_bp_kernel_of<true>(variant & (kCols - 1), f) : with_bp_kernel_of<false>(variant, f);
+    return variant & kColsMask ? with_bp_kernel_of<true>(variant & (kCols - 1), f) : with_bp_kernel_of<false>(variant, f);
 }
 
 // Multiprocessor count of the current device, cached per device ordinal (a
@@ -337,17 +346,32 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
         tall = tall && scans[i].vol.nz >= 256u;
     }
     const bool zl8 = zlanes && tall && ab_tuning_get(AB_TUNE_BP_XB) == 0;
-    // The z-column kernel for a backprojection batch only when every scan may
-    // take it (one kernel variant per plan) and some scan's views allow it.
-    bool cols = op == APRICT_BATCH_BACKPROJECT, some = false;
-    for (int i = 0; cols && i < n_scans; ++i) {
-        cols = ab_bp::bp_columns_ok(&scans[i].vol, &scans[i].projs,
-                                    static_cast<const aprict_backproject_config *>(configs) + i);
-        if (views != nullptr && views[i] > APRICT_VIEWS_GENERAL)
-            return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "scan %d: unknown view promise %u", i, views[i]);
-        some = some || views == nullptr || views[i] != APRICT_VIEWS_GENERAL;
+    // Scans that may take the z columns (view kind UPRIGHT or UNKNOWN below; the
+    // others are GENERAL whatever their views), with one XB for the plan.
+    std::vector<uint32_t> kind(n_scans, APRICT_VIEWS_GENERAL);
+    uint32_t tallest = 0;
+    uint64_t col_units = 0;
+    bool cols = false, bricks = false;
+    for (int i = 0; op == APRICT_BATCH_BACKPROJECT && i < n_scans; ++i) {
+        kind[i] = views != nullptr ? views[i] : APRICT_VIEWS_UNKNOWN;
+        if (kind[i] > APRICT_VIEWS_GENERAL)
+            return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "scan %d: unknown view promise %u", i, kind[i]);
+        if (!ab_bp::bp_columns_ok(&scans[i].vol, &scans[i].projs,
+                                  static_cast<const aprict_backproject_config *>(configs) + i))
+            kind[i] = APRICT_VIEWS_GENERAL;
+        if (kind[i] == APRICT_VIEWS_GENERAL) continue;
+        tallest = std::max(tallest, scans[i].vol.nz);
     }
-    cols = cols && some;
+    const int plan_cxb = ab_bp::col_xb(tallest);
+    for (int i = 0; i < n_scans; ++i)
+        if (kind[i] != APRICT_VIEWS_GENERAL) col_units += ab_bp::col_units_of(&scans[i].vol, plan_cxb);
+    for (int i = 0; i < n_scans; ++i) {
+        if (kind[i] != APRICT_VIEWS_GENERAL && !ab_bp::columns_pay(&scans[i].vol, static_cast<const aprict_backproject_config *>(configs) + i,
+                                                                     col_units, true))
+            kind[i] = APRICT_VIEWS_GENERAL;
+        cols = cols || kind[i] != APRICT_VIEWS_GENERAL;
+        bricks = bricks || kind[i] != APRICT_VIEWS_UPRIGHT;
+    }
     for (int i = 0; i < n_scans; ++i) {
         const aprict_scan &sc = scans[i];
         int rc;
@@ -365,15 +389,16 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
             units[i] = u;
         } else {
             const aprict_backproject_config *cfg = static_cast<const aprict_backproject_config *>(configs) + i;
-            int xb = 0, ord = -1, cxb = 8;
+            int xb = 0, ord = -1, cxb = plan_cxb;
             uint64_t u = 0, cu = 0;
             rc = ab_bp::make_bp_params(sc.specs_dev, &sc.projs, sc.projs_dev, &sc.vol, sc.vol_dev, sc.multiplier_dev,
                                        cfg, sc.status_dev, bp[i], u, xb,
                                        zl8 ? 8 : batch_xb(ab_bp::bp_ord(&sc.vol), cfg->exact != 0),
-                                       zlanes ? &ord : nullptr, cols ? &cxb : nullptr, &cu);
+                                       zlanes ? &ord : nullptr, kind[i] != APRICT_VIEWS_GENERAL ? &cxb : nullptr, &cu);
             if (rc != APRICT_OK) return scan_error(rc, i);
-            bp[i].views = views != nullptr ? (int)views[i] : (int)APRICT_VIEWS_UNKNOWN;
-            const int v = (ord == 3 ? (xb == 8 ? 16 : 15) : bp_variant(cfg, &sc.vol)) + (cols ? kCols : 0);
+            bp[i].views = (int)kind[i];
+            const int v = (ord == 3 ? (xb == 8 ? 16 : 15) : bp_variant(cfg, &sc.vol)) + (cols ? kCols * (plan_cxb / 2) : 0) +
+                          (bricks ? 0 : kNoBricks);
             if (variant >= 0 && v != variant)
                 return ab_fail(APRICT_ERR_INVALID_ARGUMENT,
                                "scan %d: every scan of a backprojection batch needs the same volume order, "
@@ -381,7 +406,8 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
                                "nearest / bilinear)",
                                i);
             variant = v;
-            units[i] = u > cu ? u : cu;  // the larger of the two kernels' (an order passes over units past its end)
+            // the larger of the two kernels' where either may run (an order passes over units past its end)
+            units[i] = kind[i] == APRICT_VIEWS_GENERAL ? u : (kind[i] == APRICT_VIEWS_UPRIGHT ? cu : std::max(u, cu));
         }
     }
     // projection variant: bit 0 = 64-bit offsets, bit 1 = sub-rays (ssu or ssv > 1)
@@ -426,7 +452,7 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
                 }
             } else {
                 rc = with_bp_kernel(variant, [&](auto k) { return grid_for(k, G->n_units, G->grid); });
-                if (rc == APRICT_OK && (variant & kCols))
+                if (rc == APRICT_OK && cols)
                     rc = with_columns_kernel(variant, [&](auto k) { return grid_for(k, G->n_units, G->col_grid); });
             }
         }
@@ -481,10 +507,10 @@ extern "C" int aprict_b200_batch_run(const void *plan_host, void *plan_dev, apri
         } else {
             using P = ab_bp::BPParams;
             rc = APRICT_OK;
-            if (H->variant & kCols)
+            if (H->variant & kColsMask)
                 rc = with_columns_kernel(H->variant,
                                          [&](auto k) { return launch_group<P>(k, gh.col_grid, gh, gd, params, st); });
-            if (rc == APRICT_OK)
+            if (rc == APRICT_OK && !(H->variant & kNoBricks))
                 rc = with_bp_kernel(H->variant, [&](auto k) { return launch_group<P>(k, gh.grid, gh, gd, params, st); });
         }
         if (rc != APRICT_OK) return rc;

@@ -1102,32 +1102,63 @@ inline bool bp_zlanes_ok(const aprict_vol_desc *vd, const aprict_proj_desc *pd, 
            !cfg->approx_mode_linear_interpolate;
 }
 
-// Host: whether a call may take the z-column kernel (ab_bpcol.cuh) when its
-// views turn out to be upright: the fast modes on a volume of more than one
-// layer, unless tuning knob 7 is 1; nearest with a v stride below 2^30
-// elements (the gathers form their byte address as a 32 x 32-bit product),
-// bilinear with v contiguous (its row pairs are gathered at one address).
+// Host: whether the z-column kernel (ab_bpcol.cuh) can take a call whose views turn
+// out to be upright: the fast modes on a volume of more than one layer, unless
+// tuning knob 7 is 1; nearest with a v stride below 2^30 elements (the gathers
+// form their byte address as a 32 x 32-bit product), bilinear with v contiguous
+// (its row pairs are gathered at one address). Whether it should: columns_pay.
 inline bool bp_columns_ok(const aprict_vol_desc *vd, const aprict_proj_desc *pd, const aprict_backproject_config *cfg) {
     return vd->nz > 1u && ab_tuning_get(AB_TUNE_BP_ZLANES) != 1 && !cfg->exact &&
            (cfg->approx_mode_linear_interpolate ? pd->stride_v == 1 && pd->stride_u < (int64_t)1 << 30
                                                 : pd->stride_v < (int64_t)1 << 30);
 }
 
-// Voxels per thread of the z-column kernel: the fewest that hold the column
-// (blocks of 32 voxels past the volume's top are skipped, but the per-view
-// work of a warp is spread over its live blocks only).
-inline int col_xb(uint32_t nz) { return nz > 128u ? 8 : (nz > 64u ? 4 : 2); }
-
-// Host: super-bricks of about one wave of `resident` CTAs per SM, with equal
-// extents in voxels along the middle (8 per block) and slowest (ext2) axes;
-// false when the units overflow a grid.
-inline bool order_bricks(BrickOrder &O, int ext2, int resident, uint64_t &units) {
+inline int bp_sms() {
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
+    return sms;
+}
+
+// Host: whether the z columns are also the faster kernel; col_units: the call's (or
+// batch's) column CTAs. A warp's table of views costs the same for a column of 2
+// voxels as for one of 32, and the lanes above a flat volume idle; the bricks put 8 x
+// 32 x 4 voxels on a view's record instead. But a volume whose columns are one wave of
+// CTAs has too few bricks to fill the GPU.
+// Measured on 256^2 x nz from 120 views, columns and bricks in us (nearest; detectors
+// that cut the volume off):
+//   C order  nz 8: 1055, 586   32: 1059, 599   40: 1180, 1122   64: 678, 1070
+//            (detectors that do not, nz 40: 656, 1005)
+//   F order  nz 8: 1061, 229   40: 1212, 748   48: 1212, 870   56: 947, 1026
+// 64^2 (one wave: 512 CTAs) x 24: 89, 126 (C), 90, 100 (F); 64^2 x 2: 88, 90 (C), 89, 83 (F).
+// Batches fill the GPU with bricks too (and skip views off a brick). 6 x 128^2 x nz:
+//   C order, nearest    nz 48: 1837, 1551   56: 1347, 1452   96: 2205, 1966
+//   C order, bilinear   nz 32: 1737, 831    48: 2531, 2988   96: 2291, 2398
+//   F order, nearest    nz 96: 2286, 2046   112: 1886, 2385
+//   F order, bilinear   nz 48: 2554, 1861   56: 1860, 2395
+inline bool columns_pay(const aprict_vol_desc *vd, const aprict_backproject_config *cfg, uint64_t col_units, bool batch) {
+    const uint64_t wave = (uint64_t)kColBlocks * (uint64_t)bp_sms();
+    if (vd->order == 0) return vd->nz > (batch ? 48u : 32u) || col_units <= wave;
+    const bool nearest = !cfg->approx_mode_direct_raycast && !cfg->approx_mode_linear_interpolate;
+    return vd->nz > (batch && nearest ? 104u : 48u) || col_units <= wave * 3 / 4;
+}
+
+// Voxels per thread of the z-column kernel: the fewest that hold the column
+// (blocks of 32 voxels past the volume's top are skipped, but the per-view
+// work of a warp is spread over its live blocks only), and its CTAs.
+inline int col_xb(uint32_t nz) { return nz > 128u ? 8 : (nz > 64u ? 4 : 2); }
+inline uint64_t col_units_of(const aprict_vol_desc *vd, int xb) {
+    return (uint64_t)((vd->nz + 32u * xb - 1u) / (32u * xb)) * ((vd->ny + 7u) / 8u) * vd->nx;
+}
+
+// Host: super-bricks of about one wave of `resident` CTAs per SM, with equal
+// extents in voxels along the middle (8 per block) and slowest (ext2) axes;
+// false when the units overflow a grid.
+inline bool order_bricks(BrickOrder &O, int ext2, int resident, uint64_t &units) {
+    const int sms = bp_sms();
     const int wave = ab_tuning_get(AB_TUNE_BP_WAVE) > 0 ? ab_tuning_get(AB_TUNE_BP_WAVE) : resident;
     const double target = (double)wave * sms / (double)O.gb[0];  // blocks of the (middle x slowest) plane per wave
     int sb1 = (int)floor(sqrt(target * ext2 / 8.0) + 0.5);

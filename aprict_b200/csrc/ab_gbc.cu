@@ -1091,6 +1091,13 @@ extern "C" int aprict_b200_backproject_gbc_views(const aprict_proj_spec *specs_d
     if (blocks > 0x7fffffffLL) return ab_fail(APRICT_ERR_TOO_LARGE, "volume too large for the grid");
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int order_f = vd->order != 0;
+    // C order: the columns at every size. F order: its lanes along x have a flat volume's
+    // voxels side by side and need no column, and a small one's are too few for 8 voxels a
+    // lane. 198^2 x nz from 120 views bilinear, columns and k_backproject_gbc: 8: 1096, 292 us;
+    // 48: 1557, 1470; 64: 791, 1971; 24^2 x 100: 164, 79; 48^2 x 64: 91, 157.
+    if (cxb != 0 && order_f &&
+        !(vd->nz > 48u && ab_bp::col_units_of(vd, kGCol) >= 3 * (uint64_t)ab_bp::bp_sms() / 2))
+        P.views = (int)(views = APRICT_VIEWS_GENERAL);
     if (cxb != 0 && views != APRICT_VIEWS_GENERAL) {
         // The window's flat part and its end as bounds on |z - s_z| / (R ell),
         // with 1e-5 to spare (the band's rule decides there); none where the

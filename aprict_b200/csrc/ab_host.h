@@ -22,13 +22,13 @@ int ab_check_projs(const aprict_proj_desc *p, const void *ptr, const char *name)
 // Launch-shape knobs (set by the autotuner through aprict_b200_set_tuning).
 enum {
     AB_TUNE_FP_TILE_V = 0,  // forward projector tile height in pixels (0 = auto, 8, 16, 32)
-    AB_TUNE_BP_XB = 1,      // backprojector voxels per thread (0 = auto = 2, 2, 4)
-    AB_TUNE_BP_WAVE = 2,    // backprojector super-brick size in CTAs per SM (0 = auto = 3)
+    AB_TUNE_BP_XB = 1,      // backprojector voxels per thread, bricks and z columns (0 = auto, 2, 4, 8)
+    AB_TUNE_BP_WAVE = 2,    // backprojector super-brick size in CTAs per SM, bricks and z columns (0 = auto)
     AB_TUNE_FP_WARP_V = 3,  // forward projector lanes of a warp along v (0 = auto = 8, 8, 16, 32)
     AB_TUNE_FP_VIEWS = 4,   // forward projector views per tile (0 = auto = 4, 1, 2, 4)
     AB_TUNE_FP_WARP_VIEWS = 5,  // forward projector views inside a warp's patch (0 = auto = 1, 1, 2, 4)
     AB_TUNE_FP_SS1 = 6,     // one-scan projector, one sub-ray per pixel: 0 = specialised path, 1 = general path
-    AB_TUNE_BP_ZLANES = 7,  // one-scan backprojector on C-order volumes: 0 = z-column layout when tall enough, 1 = never
+    AB_TUNE_BP_ZLANES = 7,  // backprojectors with lanes along z (z columns, z-lane bricks; one scan, batch, GBC): 0 = where they pay, 1 = never
     AB_TUNE_COUNT = 8
 };
 int ab_tuning_get(int key);

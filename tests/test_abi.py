@@ -231,3 +231,18 @@ def test_batch_records_keep_the_c_layout() -> None:
 
     recs = _packed([np.zeros((), S.scan)] * 3, S.scan)
     assert recs.dtype.itemsize == _lib.lib().aprict_b200_struct_size(b"aprict_scan") == 120
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+def test_batch_plan_refuses_unknown_view_promises(exact: int) -> None:
+    """Whatever the mode: also where no scan could take the kernel that the promise is for."""
+    lib = _lib.lib()
+    scans, confs = np.zeros(2, S.scan), np.zeros(2, S.backproject_config)
+    confs["exact"] = exact
+    nbytes = int(lib.aprict_b200_batch_plan_bytes(1, 2))
+    raw = np.zeros(nbytes + 256, np.uint8)
+    plan = raw[-raw.ctypes.data % 256 :]
+    views = np.array([2, 3], np.uint32)
+    rc = lib.aprict_b200_batch_plan_views(1, _lib.ptr(scans), 2, _lib.ptr(confs), _lib.ptr(views), plan.ctypes.data, nbytes)
+    assert rc == 1
+    assert b"promise" in lib.aprict_b200_last_error()

@@ -194,3 +194,36 @@ def test_many_close_rows(mode: str, nz: int) -> None:
         v = Volume.zeros(shape, voxwid=1.0)
         ScanBatch([v], [fp.ProjectionSet(pg, data=data)]).backproject(fp.ConfigBackproject(**MODES[mode]), block=True)
         np.testing.assert_array_equal(v.as_numpy(), got)
+
+
+@pytest.fixture
+def knob():
+    """Sets the z-lane knob (0 = where it pays, 1 = never)."""
+    from aprict_b200 import _lib, autotune
+
+    lib = _lib.lib()
+    yield lambda value: _lib.check(lib.aprict_b200_set_tuning(autotune.KEY_BP_ZLANES, value), "set_tuning")
+    lib.aprict_b200_set_tuning(autotune.KEY_BP_ZLANES, 0)
+
+
+@pytest.mark.parametrize("order", ["C", "F"])
+@pytest.mark.parametrize("mode", ["nearest-taper", "bilinear", "raycast"])
+def test_flat_volumes_on_both_sides_of_the_rule(mode: str, order: str, knob) -> None:  # noqa: ANN001
+    """Volumes of more columns than one wave of CTAs: flat ones take the bricks, tall ones the columns; at every
+    height the call gives what either kernel gives, alone and in a batch with others of other kinds."""
+    shapes = [(90, 71, nz) for nz in (2, 31, 32, 33, 48, 49)]
+    pgs = [circular(10, 300, 200, 1.37, 77, max(12, int(0.9 * s[2]))) for s in shapes]
+    datas = [_data(g, i) for i, g in enumerate(pgs)]
+    tol = 1e-5 if mode == "bilinear" else 1e-6
+    auto, bricks = [], []
+    for value, out in ((0, auto), (1, bricks)):
+        knob(value)
+        out.extend(_run(mode, g, d, s, order) for s, g, d in zip(shapes, pgs, datas))
+    knob(0)
+    vols = [Volume.zeros(s, voxwid=1.0, order=order) for s in shapes]
+    ScanBatch(vols, [fp.ProjectionSet(g, data=d) for g, d in zip(pgs, datas)]).backproject(
+        fp.ConfigBackproject(**MODES[mode]), block=True)
+    for a, b, v in zip(auto, bricks, vols):
+        assert np.linalg.norm(b) > 0
+        assert rel_l2(a, b) <= tol
+        assert rel_l2(v.as_numpy(), b) <= tol

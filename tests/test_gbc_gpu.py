@@ -273,3 +273,27 @@ def test_gbc_reconstruction_matches_oracle() -> None:
     assert got.shape == want.shape == (n_vox,) * 3
     assert np.linalg.norm(want) > 0
     assert rel_l2(got, want) <= 1e-4
+
+
+@pytest.mark.parametrize("linear", [False, True])
+@pytest.mark.parametrize("order", ["C", "F"])
+@pytest.mark.parametrize("shape", [(12, 11, 9), (40, 40, 48), (40, 40, 49), (50, 48, 49), (50, 48, 40)])
+def test_every_kernel_gives_the_same(shape: tuple, order: str, linear: bool) -> None:
+    """F-order volumes take the columns above 48 layers and 222 CTAs, C-order ones at every size: without a promise,
+    with it, and with the general kernel, all to FP32 rounding (bilinear: the general kernels' coordinates are FP32); a scan with one tilted view takes the general kernel also without a promise."""
+    pg = _scan(m=20, h=8.0, nu=61, nv=50)
+    vecs = {k: np.broadcast_to(getattr(pg, k), (20, 3)).copy() for k in ("source_pos", "det_pos", "det_uvec", "det_vvec")}
+    vecs["det_vvec"][5] += 0.01 * vecs["det_uvec"][5]
+    projs = np.random.default_rng(7).random((20, 61, 50)).astype(np.float32)
+    for g, forms in ((pg, (0, 1, 2)), (fp.ProjGeom(**vecs, nu=pg.nu, nv=pg.nv), (0, 2))):
+        out = []
+        for views in forms:
+            v, ws = Volume.zeros(shape, voxwid=0.9, order=order), Volume.zeros(shape, voxwid=0.9, order=order)
+            ps = fp.ProjectionSet(g, data=projs)
+            ps._backproject_promise = lambda needs_z, views=views: views  # noqa: SLF001
+            fp.backproject(_cfg(linear), v, ps, secondary_volume=ws, block=True)
+            out.append((v.as_numpy(), ws.as_numpy()))
+        assert np.linalg.norm(out[-1][0]) > 0
+        for a, w in out[:-1]:
+            assert rel_l2(a, out[-1][0]) <= 1e-5
+            assert rel_l2(w, out[-1][1]) <= 1e-6
