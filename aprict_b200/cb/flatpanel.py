@@ -376,7 +376,7 @@ class ProjectionSet:
         self._proj_specs = proj_specs
         self._data = data
         self._specs_dev: torch.Tensor | None = None
-        self._kinds: tuple[bool, bool] | None = None
+        self._kinds: tuple[int, int] | None = None
         self._out_of_mem_counter: torch.Tensor | None = None
 
     def _with_data(self, data: torch.Tensor) -> ProjectionSet:
@@ -441,9 +441,9 @@ class ProjectionSet:
         if self._kinds is None:
             sp = self._proj_specs
             up = (sp["det_u"]["z"] == 0) & (sp["det_v"]["x"] == 0) & (sp["det_v"]["y"] == 0)
-            self._kinds = (bool(up.all()), bool((sp["det_pos"]["z"] == sp["source_pos"]["z"]).all()))
-        upright, level = self._kinds
-        return 1 if upright and (level or not needs_z) else 2
+            level = up & (sp["det_pos"]["z"] == sp["source_pos"]["z"])
+            self._kinds = tuple(1 if k.all() else 3 if k.any() else 2 for k in (up, level))
+        return self._kinds[bool(needs_z)]
 
     def create_buffer(self, *, dtype: type | np.dtype = np.float32, existing_ok: bool = False) -> None:
         """Allocate a zero-filled data buffer."""

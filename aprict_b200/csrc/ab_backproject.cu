@@ -8,13 +8,13 @@ namespace {
 
 using namespace ab_bp;
 
-template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, int XB>
+template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, int XB, bool ZT = false>
 __global__ void __launch_bounds__(kThreads, bp_min_blocks(XB, EXACT)) k_backproject(const BPParams P) {
-    __shared__ BPSmem<EXACT, BILIN, XB> sm;
+    __shared__ BPSmem<EXACT, BILIN, XB, ZT> sm;
     if constexpr (!EXACT && ORD != 2) {
         if (P.views == (int)APRICT_VIEWS_UNKNOWN && P.col.gb[0] != 0 && all_upright(P)) return;  // k_backproject_columns'
     }
-    bp_brick<ORD, EXACT, RAYCAST, BILIN, XB>(P, blockIdx.x, sm);
+    bp_brick<ORD, EXACT, RAYCAST, BILIN, XB, RAYCAST, ZT>(P, blockIdx.x, sm);
 }
 
 template <bool RAYCAST, bool BILIN, int XB>
@@ -49,6 +49,8 @@ void launch_bp(const BPParams &P, const aprict_backproject_config *cfg, bool lin
         }
     } else if (lin) {
         if constexpr (ORD != 3) k_backproject<ORD, false, false, true, XB><<<grid, kThreads, 0, st>>>(P);
+    } else if (ORD == 3 && P.views != (int)APRICT_VIEWS_GENERAL) {  // some views may be upright
+        k_backproject<ORD, false, false, false, XB, ORD == 3><<<grid, kThreads, 0, st>>>(P);
     } else {
         k_backproject<ORD, false, false, false, XB><<<grid, kThreads, 0, st>>>(P);
     }
@@ -60,7 +62,7 @@ extern "C" int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev, 
                                              const float *projs_dev, const aprict_vol_desc *vd, float *vol_dev,
                                              const float *multiplier_dev, const aprict_backproject_config *cfg,
                                              uint32_t views, uint32_t *status_dev, aprict_stream_t stream) {
-    if (views > APRICT_VIEWS_GENERAL)
+    if (views > APRICT_VIEWS_MIXED)
         return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "backproject: unknown view promise %u", views);
     BPParams P;
     uint64_t grid = 0, col_grid = 0;
@@ -74,8 +76,8 @@ extern "C" int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev, 
     P.views = (int)views;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const bool lin = cfg->approx_mode_linear_interpolate != 0;
-    if (cxb != 0 && !columns_pay(vd, cfg, col_units_of(vd, cxb), false)) P.views = (int)(views = APRICT_VIEWS_GENERAL);
-    if (cxb != 0 && views != APRICT_VIEWS_GENERAL) {
+    if (cxb != 0 && views != APRICT_VIEWS_MIXED && !columns_pay(vd, cfg, col_units_of(vd, cxb), false)) P.views = (int)(views = APRICT_VIEWS_GENERAL);
+    if (cxb != 0 && (views == APRICT_VIEWS_UNKNOWN || views == APRICT_VIEWS_UPRIGHT)) {
         const bool ray = cfg->approx_mode_direct_raycast != 0;
         if (cxb == 8)
             launch_columns<8>(P, ray, lin, (unsigned)col_grid, st);

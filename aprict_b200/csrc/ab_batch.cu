@@ -150,15 +150,16 @@ constexpr int batch_xb(int ord, bool exact) { return ord == 2 ? 4 : ab_bp::defau
 // the helical ones leave most of a volume off each view's detector (48
 // uneven scans: 326.6 -> 265.3 ms per batched backprojection).
 // COLS: leave the scans that take the z columns to k_batch_columns.
-template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, bool COLS, int XB = batch_xb(ORD, EXACT)>
+// ZT: the table of the z-lane layout's upright views (bp_brick).
+template <int ORD, bool EXACT, bool RAYCAST, bool BILIN, bool COLS, int XB = batch_xb(ORD, EXACT), bool ZT = false>
 __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::bp_min_blocks(XB, EXACT))
     k_batch_backproject(const __grid_constant__ BatchArgs<ab_bp::BPParams> A) {
-    __shared__ ab_bp::BPSmem<EXACT, BILIN, XB> sm;
+    __shared__ ab_bp::BPSmem<EXACT, BILIN, XB, ZT> sm;
     uint32_t unit;
     int s;
     while (next_unit(A, unit, s)) {
         if (COLS && ab_bp::all_upright(A.scans[s])) continue;
-        ab_bp::bp_brick<ORD, EXACT, RAYCAST, BILIN, XB, true>(A.scans[s], unit, sm);
+        ab_bp::bp_brick<ORD, EXACT, RAYCAST, BILIN, XB, true, ZT>(A.scans[s], unit, sm);
     }
     retire(A.g);
 }
@@ -183,7 +184,8 @@ __global__ void __launch_bounds__(ab_bp::kThreads, ab_bp::kColBlocks)
 // Backprojection kernel variant code: ORD + 3 * mode (ORD from ab_bp::bp_ord),
 // mode 0 fast nearest, 1 fast bilinear, 2 raycast nearest, 3 raycast
 // bilinear, 4 exact; 15: fast nearest in the z-lane layout (ORD 3) with 4
-// voxels per thread, 16: the same with 8 (every scan at least 256 voxels tall).
+// voxels per thread, 16: the same with 8 (every scan at least 256 voxels tall); 17,
+// 18: those two with the table of upright views (some scan may have some).
 // kCols times 1, 2 or 4 (the columns' XB 2, 4 or 8) is added where scans may take the
 // z columns, kNoBricks where all are promised to.
 constexpr int kCols = 32, kColsMask = 7 * kCols, kNoBricks = 256;
@@ -196,8 +198,10 @@ int bp_variant(const aprict_backproject_config *c, const aprict_vol_desc *vd) {
 // The batch backprojection kernel of a variant code.
 template <int V, bool COLS>
 auto bp_kernel() {
-    if constexpr (V == 16) {
-        return k_batch_backproject<3, false, false, false, COLS, 8>;
+    if constexpr (V == 17) {
+        return k_batch_backproject<3, false, false, false, COLS, batch_xb(3, false), true>;
+    } else if constexpr (V == 16 || V == 18) {
+        return k_batch_backproject<3, false, false, false, COLS, 8, V == 18>;
     } else {
         constexpr int ORD = V == 15 ? 3 : V % 3, mode = V == 15 ? 0 : V / 3;
         // one-layer volumes and the exact mode have no columns
@@ -206,7 +210,7 @@ auto bp_kernel() {
     }
 }
 
-// The z-column kernel of a variant code's mode (15 and 16 are mode 0).
+// The z-column kernel of a variant code's mode (15 and above are mode 0).
 template <int XB, class F>
 int with_columns_kernel_of(int v, F &&f) {
     switch (v < 15 ? v / 3 : 0) {
@@ -247,6 +251,8 @@ int with_bp_kernel_of(int variant, F &&f) {
         case 14: return f(bp_kernel<14, COLS>());
         case 15: return f(bp_kernel<15, COLS>());
         case 16: return f(bp_kernel<16, COLS>());
+        case 17: return f(bp_kernel<17, COLS>());
+        case 18: return f(bp_kernel<18, COLS>());
         default: return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "corrupt batch plan (variant %d)", variant);
     }
 }
@@ -346,30 +352,31 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
         tall = tall && scans[i].vol.nz >= 256u;
     }
     const bool zl8 = zlanes && tall && ab_tuning_get(AB_TUNE_BP_XB) == 0;
-    // Scans that may take the z columns (view kind UPRIGHT or UNKNOWN below; the
-    // others are GENERAL whatever their views), with one XB for the plan.
+    // Scans that may take the z columns keep view kind UPRIGHT or UNKNOWN (the
+    // others become GENERAL whatever their views), with one XB for the plan.
     std::vector<uint32_t> kind(n_scans, APRICT_VIEWS_GENERAL);
+    auto col = [&](int i) { return kind[i] == APRICT_VIEWS_UPRIGHT || kind[i] == APRICT_VIEWS_UNKNOWN; };
     uint32_t tallest = 0;
     uint64_t col_units = 0;
-    bool cols = false, bricks = false;
+    bool cols = false, bricks = false, ztable = false;
     for (int i = 0; op == APRICT_BATCH_BACKPROJECT && i < n_scans; ++i) {
         kind[i] = views != nullptr ? views[i] : APRICT_VIEWS_UNKNOWN;
-        if (kind[i] > APRICT_VIEWS_GENERAL)
+        if (kind[i] > APRICT_VIEWS_MIXED)
             return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "scan %d: unknown view promise %u", i, kind[i]);
-        if (!ab_bp::bp_columns_ok(&scans[i].vol, &scans[i].projs,
-                                  static_cast<const aprict_backproject_config *>(configs) + i))
+        ztable = ztable || kind[i] == APRICT_VIEWS_MIXED || kind[i] == APRICT_VIEWS_UNKNOWN;
+        if (col(i) && !ab_bp::bp_columns_ok(&scans[i].vol, &scans[i].projs,
+                                            static_cast<const aprict_backproject_config *>(configs) + i))
             kind[i] = APRICT_VIEWS_GENERAL;
-        if (kind[i] == APRICT_VIEWS_GENERAL) continue;
-        tallest = std::max(tallest, scans[i].vol.nz);
+        if (col(i)) tallest = std::max(tallest, scans[i].vol.nz);
     }
     const int plan_cxb = ab_bp::col_xb(tallest);
     for (int i = 0; i < n_scans; ++i)
-        if (kind[i] != APRICT_VIEWS_GENERAL) col_units += ab_bp::col_units_of(&scans[i].vol, plan_cxb);
+        if (col(i)) col_units += ab_bp::col_units_of(&scans[i].vol, plan_cxb);
     for (int i = 0; i < n_scans; ++i) {
-        if (kind[i] != APRICT_VIEWS_GENERAL && !ab_bp::columns_pay(&scans[i].vol, static_cast<const aprict_backproject_config *>(configs) + i,
-                                                                     col_units, true))
+        if (col(i) && !ab_bp::columns_pay(&scans[i].vol, static_cast<const aprict_backproject_config *>(configs) + i,
+                                          col_units, true))
             kind[i] = APRICT_VIEWS_GENERAL;
-        cols = cols || kind[i] != APRICT_VIEWS_GENERAL;
+        cols = cols || col(i);
         bricks = bricks || kind[i] != APRICT_VIEWS_UPRIGHT;
     }
     for (int i = 0; i < n_scans; ++i) {
@@ -394,10 +401,10 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
             rc = ab_bp::make_bp_params(sc.specs_dev, &sc.projs, sc.projs_dev, &sc.vol, sc.vol_dev, sc.multiplier_dev,
                                        cfg, sc.status_dev, bp[i], u, xb,
                                        zl8 ? 8 : batch_xb(ab_bp::bp_ord(&sc.vol), cfg->exact != 0),
-                                       zlanes ? &ord : nullptr, kind[i] != APRICT_VIEWS_GENERAL ? &cxb : nullptr, &cu);
+                                       zlanes ? &ord : nullptr, col(i) ? &cxb : nullptr, &cu);
             if (rc != APRICT_OK) return scan_error(rc, i);
             bp[i].views = (int)kind[i];
-            const int v = (ord == 3 ? (xb == 8 ? 16 : 15) : bp_variant(cfg, &sc.vol)) + (cols ? kCols * (plan_cxb / 2) : 0) +
+            const int v = (ord == 3 ? (xb == 8 ? 16 : 15) + (ztable ? 2 : 0) : bp_variant(cfg, &sc.vol)) + (cols ? kCols * (plan_cxb / 2) : 0) +
                           (bricks ? 0 : kNoBricks);
             if (variant >= 0 && v != variant)
                 return ab_fail(APRICT_ERR_INVALID_ARGUMENT,
@@ -407,7 +414,7 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
                                i);
             variant = v;
             // the larger of the two kernels' where either may run (an order passes over units past its end)
-            units[i] = kind[i] == APRICT_VIEWS_GENERAL ? u : (kind[i] == APRICT_VIEWS_UPRIGHT ? cu : std::max(u, cu));
+            units[i] = !col(i) ? u : (kind[i] == APRICT_VIEWS_UPRIGHT ? cu : std::max(u, cu));
         }
     }
     // projection variant: bit 0 = 64-bit offsets, bit 1 = sub-rays (ssu or ssv > 1)

@@ -1056,7 +1056,8 @@ extern "C" int aprict_b200_backproject_gbc_views(const aprict_proj_spec *specs_d
                                                  float *weightsum_dev, const float *multiplier_dev,
                                                  const aprict_backproject_config *cfg, uint32_t views, uint32_t *status_dev,
                                                  aprict_stream_t stream) {
-    if (views > APRICT_VIEWS_GENERAL) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "GBC: unknown view promise %u", views);
+    if (views > APRICT_VIEWS_MIXED) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "GBC: unknown view promise %u", views);
+    if (views == APRICT_VIEWS_MIXED) views = APRICT_VIEWS_GENERAL;  // one kernel for both
     if (cfg == nullptr) return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "null backproject config");
     if (cfg->weighting_preset != 7)
         return ab_fail(APRICT_ERR_INVALID_ARGUMENT, "the GBC backprojection takes weighting preset 7");

@@ -193,11 +193,15 @@ APRICT_API int aprict_b200_backproject(const aprict_proj_spec *specs_dev,
  * height); calls whose views are all upright have a faster kernel. Without a
  * promise both kernels are launched and each looks at the views itself.
  *   views: APRICT_VIEWS_UNKNOWN, APRICT_VIEWS_UPRIGHT (a promise: the result is
- *          undefined if a view is not upright) or APRICT_VIEWS_GENERAL (the
- *          general kernel whatever the views)                              */
+ *          undefined if a view is not upright), APRICT_VIEWS_GENERAL (the
+ *          general kernel, in the form for scans with no upright view) or
+ *          APRICT_VIEWS_MIXED (the general kernel, in the form for scans with
+ *          views of both kinds); the last two give the same results whatever
+ *          the views                                                       */
 #define APRICT_VIEWS_UNKNOWN 0u
 #define APRICT_VIEWS_UPRIGHT 1u
 #define APRICT_VIEWS_GENERAL 2u
+#define APRICT_VIEWS_MIXED 3u
 APRICT_API int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev,
                                   const aprict_proj_desc *projs,
                                   const float *projs_dev,

@@ -242,7 +242,7 @@ def test_batch_plan_refuses_unknown_view_promises(exact: int) -> None:
     nbytes = int(lib.aprict_b200_batch_plan_bytes(1, 2))
     raw = np.zeros(nbytes + 256, np.uint8)
     plan = raw[-raw.ctypes.data % 256 :]
-    views = np.array([2, 3], np.uint32)
+    views = np.array([2, 4], np.uint32)
     rc = lib.aprict_b200_batch_plan_views(1, _lib.ptr(scans), 2, _lib.ptr(confs), _lib.ptr(views), plan.ctypes.data, nbytes)
     assert rc == 1
     assert b"promise" in lib.aprict_b200_last_error()

@@ -227,3 +227,37 @@ def test_flat_volumes_on_both_sides_of_the_rule(mode: str, order: str, knob) -> 
         assert np.linalg.norm(b) > 0
         assert rel_l2(a, b) <= tol
         assert rel_l2(v.as_numpy(), b) <= tol
+
+
+@pytest.mark.parametrize("nz", [64, 130, 260])
+@pytest.mark.parametrize("mode", ["nearest-taper", "nearest-z"])
+def test_mixed_scans_on_tall_volumes(mode: str, nz: int) -> None:
+    """A scan with views of both kinds on a volume of z-lane bricks (4 and 8 voxels per thread, and below them): known
+    to be mixed, nothing known, and the form without the table of upright views; alone and in batches."""
+    cfg = dict(MODES["nearest-taper"], cyl_mask_rad=5.0) if mode == "nearest-taper" else dict(fast_approx=True, Z_on_val_factor_power=-1, Z_on_val_factor_val=100.0)
+    pg = circular(70, 200, 160, 0.913, 25, nz - 20, theta0=0.3)
+    tilted = jittered(np.random.default_rng(2), pg)
+    vecs = {k: np.broadcast_to(getattr(pg, k), (70, 3)).copy() for k in ("source_pos", "det_pos", "det_uvec", "det_vvec")}
+    for k in vecs:
+        vecs[k][[3, 40, 41, 69]] = getattr(tilted, k)[[3, 40, 41, 69]]
+    g, shape = fp.ProjGeom(**vecs, nu=pg.nu, nv=pg.nv), (9, 11, nz)
+    data = _data(g, nz)
+    conf = fp.ConfigBackproject(**cfg)
+    want = O.backproject(g.to_proj_spec_array(), data.cpu().numpy(), shape, conf.contents, voxwid=1.0,
+                         corner=-np.array(shape, np.float32) / 2)
+    assert fp.ProjectionSet(g, data=data)._backproject_promise(conf.needs_z) == 3
+    out = []
+    for views in (3, 0, 2):
+        v, ps = Volume.zeros(shape, voxwid=1.0), fp.ProjectionSet(g, data=data)
+        ps._backproject_promise = lambda needs_z, views=views: views  # noqa: SLF001
+        fp.backproject(conf, v, ps, block=True)
+        out.append(v.as_numpy())
+        assert rel_l2(out[-1], want) <= 1e-5
+    np.testing.assert_array_equal(out[0], out[1])
+    geoms = [g, pg, tilted]
+    vols = [Volume.zeros(shape, voxwid=1.0) for _ in geoms]
+    ScanBatch(vols, [fp.ProjectionSet(k, data=data) for k in geoms]).backproject(conf, block=True)
+    for k, v in zip(geoms, vols):
+        one = Volume.zeros(shape, voxwid=1.0)
+        fp.backproject(conf, one, fp.ProjectionSet(k, data=data), block=True)
+        assert rel_l2(v.as_numpy(), one.as_numpy()) <= 1e-6
