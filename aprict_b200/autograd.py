@@ -49,7 +49,8 @@ class SiddonProjector:
         """A x (no autograd)."""
         out = torch.zeros(self.data_shape, dtype=torch.float32, device=x.device)
         ps = fp.ProjectionSet(self.pg, data=out)
-        ps._specs_dev = self._ps.specs_device()  # noqa: SLF001
+        self._ps.specs_device()
+        ps._share_views(self._ps)  # noqa: SLF001
         fp.project(self.config, self._volume(x), ps)
         return out
 
@@ -57,7 +58,8 @@ class SiddonProjector:
         """A^T y (no autograd), the exact transpose of :meth:`forward_raw`."""
         out = torch.zeros(self.shape, dtype=torch.float32, device=y.device)
         ps = fp.ProjectionSet(self.pg, data=y.contiguous())
-        ps._specs_dev = self._ps.specs_device()  # noqa: SLF001
+        self._ps.specs_device()
+        ps._share_views(self._ps)  # noqa: SLF001
         fp.backproject_adjoint(self.config, Volume.from_tensor(out, voxwid=self.voxwid, pos_c=self.pos_c), ps)
         return out
 

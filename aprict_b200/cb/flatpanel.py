@@ -376,6 +376,7 @@ class ProjectionSet:
         self._proj_specs = proj_specs
         self._data = data
         self._specs_dev: torch.Tensor | None = None
+        self._specs_host: np.ndarray | None = None
         self._kinds: tuple[int, int] | None = None
         self._out_of_mem_counter: torch.Tensor | None = None
 
@@ -387,10 +388,14 @@ class ProjectionSet:
         out._proj_geom = self._proj_geom
         out._proj_specs = self._proj_specs
         out._data = data
-        out._specs_dev = self.specs_device()
-        out._kinds = self._kinds
+        self.specs_device()
+        out._share_views(self)
         out._out_of_mem_counter = None
         return out
+
+    def _share_views(self, other: ProjectionSet) -> None:
+        """Take over what ``other``, a set of the same geometry, has uploaded of its views."""
+        self._specs_dev, self._specs_host, self._kinds = other._specs_dev, other._specs_host, other._kinds
 
     @property
     def proj_geom(self) -> ProjGeom:
@@ -431,15 +436,16 @@ class ProjectionSet:
     def specs_device(self) -> torch.Tensor:
         """The packed views on the device (uint8 bytes, flattened), cached."""
         if self._specs_dev is None:
-            raw = np.ascontiguousarray(self._proj_specs.reshape(-1)).view(np.uint8)
+            self._specs_host = self._proj_specs.reshape(-1).copy()
             _device()
-            self._specs_dev = _lib.upload(raw)
+            self._specs_dev = _lib.upload(self._specs_host.view(np.uint8))
         return self._specs_dev
 
     def _backproject_promise(self, needs_z: bool) -> int:
-        """What the packed views let a backprojection promise (``aprict_b200_backproject_views``)."""
+        """What the device's views let a backprojection promise (``aprict_b200_backproject_views``)."""
         if self._kinds is None:
-            sp = self._proj_specs
+            self.specs_device()
+            sp = self._specs_host  # as uploaded
             up = (sp["det_u"]["z"] == 0) & (sp["det_v"]["x"] == 0) & (sp["det_v"]["y"] == 0)
             level = up & (sp["det_pos"]["z"] == sp["source_pos"]["z"])
             self._kinds = tuple(1 if k.all() else 3 if k.any() else 2 for k in (up, level))
@@ -464,7 +470,7 @@ class ProjectionSet:
             msg = "Cannot create a zeroed copy without an explicit 'dtype' argument, because the object you are trying to copy does not yet have a determined dtype."
             raise ValueError(msg)
         ps = ProjectionSet(self._proj_geom, data=None)
-        ps._specs_dev, ps._kinds = self._specs_dev, self._kinds
+        ps._share_views(self)
         ps.create_buffer(dtype=_np_dtype(self._data) if dtype is None else dtype)
         return ps
 
@@ -598,7 +604,7 @@ def _f32_twin(projs: ProjectionSet) -> ProjectionSet:
     if projs.data.dtype == torch.float32:
         return projs
     tw = ProjectionSet(projs.proj_geom, data=torch.zeros(projs.data.shape, dtype=torch.float32, device=projs.data.device))
-    tw._specs_dev, tw._kinds = projs._specs_dev, projs._kinds  # noqa: SLF001
+    tw._share_views(projs)  # noqa: SLF001
     tw._out_of_mem_counter = projs.out_of_mem_counter  # noqa: SLF001
     return tw
 

@@ -261,3 +261,21 @@ def test_mixed_scans_on_tall_volumes(mode: str, nz: int) -> None:
         one = Volume.zeros(shape, voxwid=1.0)
         fp.backproject(conf, one, fp.ProjectionSet(k, data=data), block=True)
         assert rel_l2(v.as_numpy(), one.as_numpy()) <= 1e-6
+
+
+def test_promise_is_of_the_uploaded_views() -> None:
+    """The views' kind is that of the records on the device, whatever became of the host's since."""
+    shape = (12, 11, 64)
+    pg = jittered(np.random.default_rng(5), circular(9, 120, 100, 0.713, 26, 60))
+    data = _data(pg, 1)
+    want = _run("nearest", pg, data, shape)
+    assert np.linalg.norm(want) > 0
+    ps = fp.ProjectionSet(pg, data=data.clone())
+    fp.project(fp.ConfigProject(), Volume.zeros(shape, voxwid=1.0), ps)  # uploads the views, adds nothing
+    sp = ps.proj_specs
+    sp["det_u"]["z"] = sp["det_v"]["x"] = sp["det_v"]["y"] = 0
+    for p in (ps, ps._with_data(data), ps.zeroed_copy()):
+        assert p._backproject_promise(False) == 2
+    v = Volume.zeros(shape, voxwid=1.0)
+    fp.backproject(fp.ConfigBackproject(**MODES["nearest"]), v, ps, block=True)
+    np.testing.assert_array_equal(v.as_numpy(), want)
