@@ -118,7 +118,9 @@ def _one_scan_stack(projs: list[fp.ProjectionSet], volumes: list[Volume]) -> boo
     if not (sp.ndim == 1 and np.all(sp["nv"] == 1) and np.all(sp["det_u"]["z"] == 0) and np.all(sp["det_v"]["x"] == 0)
             and np.all(sp["det_v"]["y"] == 0) and np.all(sp["source_pos"]["z"] == z) and np.all(sp["det_pos"]["z"] == z)):
         return False
-    if any(p.proj_geom is not projs[0].proj_geom and not np.array_equal(p.proj_specs, sp) for p in projs):
+    # the packed views, not the geometry they came from: that may have changed since one of them was packed
+    packed = sp.tobytes()
+    if any(p.proj_specs.dtype != sp.dtype or p.proj_specs.tobytes() != packed for p in projs[1:]):
         return False
     pos = v0.pos_c
     return v0.shape[2] == 1 and all(

@@ -94,11 +94,15 @@ def test_batched_slices_equal_single_slice_fbp() -> None:
 
 @pytest.mark.parametrize(("slices", "n", "nu"), [(4, 40, 90), (5, 33, 128), (9, 50, 200), (17, 21, 96), (33, 70, 150),
                                                  (64, 24, 140), (67, 20, 130)])
-def test_slice_stack_equals_single_slices(slices: int, n: int, nu: int) -> None:
+def test_slice_stack_equals_single_slices(slices: int, n: int, nu: int, monkeypatch: pytest.MonkeyPatch) -> None:
     """Stacks of one scan run through the interleaved kernel: slice counts around its lane groups (4 slices
     a lane, 1 to 16 lanes) and past one call's 64, slices narrower than a tile, rows filtered directly
     (nu < 128) and by FFT. Each slice equals its own reconstruction up to FP32 rounding."""
+    from aprict_b200 import recon
     from aprict_b200.recon import fbp_fan_circ_batch
+
+    calls, stack = [], recon._backproject_slices  # noqa: SLF001
+    monkeypatch.setattr(recon, "_backproject_slices", lambda *a: (calls.append(len(a[3])), stack(*a)))
 
     pg = circular(75, 120.0, 100.0, 0.9 * n * 0.5 / nu * 1.2345, nu, 1, theta0=0.21)
     rng = np.random.default_rng(slices)
@@ -112,14 +116,21 @@ def test_slice_stack_equals_single_slices(slices: int, n: int, nu: int) -> None:
         vols.append(Volume.zeros((n, n + 3, 1), voxwid=0.5))
         vols[-1].fill(0.25)  # added to
     fbp_fan_circ_batch(projs, vols)
+    assert sum(calls) == slices
     for v, w in zip(vols, want):
         assert np.linalg.norm(w) > 0
         assert rel_l2(v.as_numpy() - 0.25, w) <= 2e-6
 
 
-@pytest.mark.parametrize("case", ["off plane", "other views", "F order", "other grid", "bilinear"])
-def test_slice_stacks_that_do_not_share_a_scan_go_one_by_one(case: str) -> None:
+@pytest.mark.parametrize("case", ["off plane", "other views", "changed geometry", "F order", "other grid", "bilinear"])
+def test_slice_stacks_that_do_not_share_a_scan_go_one_by_one(case: str, monkeypatch: pytest.MonkeyPatch) -> None:
+    from aprict_b200 import recon
     from aprict_b200.recon import fbp_fan_circ_batch
+
+    def stacked(*_: object) -> None:
+        pytest.fail("backprojected as a stack of one scan")
+
+    monkeypatch.setattr(recon, "_backproject_slices", stacked)
 
     n, nu = 40, 130
     pgs = [circular(60, 120.0, 100.0, 0.21, nu, 1, theta0=0.21) for _ in range(5)]
@@ -133,11 +144,22 @@ def test_slice_stacks_that_do_not_share_a_scan_go_one_by_one(case: str) -> None:
     elif case == "off plane":
         z = 0.05
     rng = np.random.default_rng(3)
-    projs = [fp.ProjectionSet(g, data=rng.random((60, nu, 1)).astype(np.float32)) for g in pgs]
+    if case == "changed geometry":  # one object, turned by a view after some of the sets were made
+        pgs = [pgs[0]] * 5
+    projs = []
+    for i, g in enumerate(pgs):
+        if case == "changed geometry" and i == 3:
+            for k in ("source_pos", "det_pos", "det_uvec"):
+                a = getattr(g, k)
+                a[...] = np.roll(a, 7, axis=0)
+        projs.append(fp.ProjectionSet(g, data=rng.random((60, nu, 1)).astype(np.float32)))
     vols = [Volume.zeros(s, voxwid=0.5, order=order, pos_c=(0, 0, z)) for s in shapes]
     fbp_fan_circ_batch(projs, vols, interpolate=case == "bilinear")
-    for p, s, v in zip(projs, shapes, vols):
+    rolled = [fp.ProjGeom(**{k: np.roll(np.broadcast_to(getattr(g, k), (60, 3)), -7, axis=0) for k in
+                             ("source_pos", "det_pos", "det_uvec")}, det_vvec=g.det_vvec, nu=g.nu, nv=g.nv)
+              if case == "changed geometry" and i < 3 else g for i, g in enumerate(pgs)]
+    for p, g, s, v in zip(projs, rolled, shapes, vols):
         one = Volume.zeros(s, voxwid=0.5, order=order, pos_c=(0, 0, z))
-        fbp_fan_circ(p, one, interpolate=case == "bilinear")
+        fbp_fan_circ(fp.ProjectionSet(g, data=p.data), one, interpolate=case == "bilinear")
         # (bilinear coordinates are stepped in FP32 from the thread's first voxel, two voxels against four)
         assert rel_l2(v.as_numpy(), one.as_numpy()) <= (2e-5 if case == "bilinear" else 2e-6)
