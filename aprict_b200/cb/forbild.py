@@ -65,6 +65,17 @@ def _compiled(volume: object) -> _Compiled:
     return volume._compiled[1]
 
 
+def _scratch(nbytes: int, least: int, device: torch.device) -> torch.Tensor | None:
+    """Device scratch of ``nbytes``, or what is to be had of it from ``least`` up (the projector
+    takes the views in groups then), or none (its tiles derive the records themselves)."""
+    while nbytes >= max(1, least):
+        try:
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        except torch.cuda.OutOfMemoryError:
+            nbytes //= 4
+    return None
+
+
 def project_shapes(config: object, volume: object, projs: object) -> None:
     """Accumulate the analytic projection of ``volume`` (an FBVolume) into ``projs``."""
     from .flatpanel import _leading_slices, _stream, _view_args  # noqa: PLC0415
@@ -79,14 +90,15 @@ def project_shapes(config: object, volume: object, projs: object) -> None:
         mode = 0
     counter = projs.out_of_mem_counter
     lib = _lib.lib()
-    nbytes = int(lib.aprict_b200_project_forbild_scratch_bytes(int(projs.proj_specs.shape[-1]), comp.n))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=comp.dev.device)
+    size = lib.aprict_b200_project_forbild_scratch_bytes
+    scratch = _scratch(int(size(int(projs.proj_specs.shape[-1]), comp.n)), int(size(1, comp.n)), comp.dev.device)
+    sptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
     for it, first in _leading_slices(projs):
         specs, pd, dptr = _view_args(projs, it, first)
         _lib.check(
             lib.aprict_b200_project_forbild_scratch(
                 specs, _lib.ptr(pd), dptr, comp.dev.data_ptr(), comp.n, float(cfg["multiply_before_adding"]),
-                int(cfg["ssu"]), int(cfg["ssv"]), mode, counter.data_ptr(), None, scratch.data_ptr() or None, nbytes,
+                int(cfg["ssu"]), int(cfg["ssv"]), mode, counter.data_ptr(), None, sptr, nbytes,
                 _stream(),
             ),
             "project (FORBILD)",

@@ -295,3 +295,29 @@ def test_gpu_around_one_chunk(n: int) -> None:
     got, _ = _gpu_project(shapes, pg, ssu=2, ssv=2)
     want = O.project_forbild(pg.to_proj_spec_array(), shapes, mode=0, ssu=2, ssv=2)
     assert rel_l2(got, want) <= 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("views", [0, 1, 4, 6])
+def test_gpu_projects_when_memory_is_short(views: int, monkeypatch: pytest.MonkeyPatch) -> None:
+    """Scratch for all 18 views' records not to be had, only some views' or none: the same projections."""
+    import torch
+
+    from aprict_b200 import _lib
+
+    shapes = random_shapes_all_types(np.random.default_rng(4), 30)
+    pg = circular(18, 150, 150, 0.5, 40, 33)
+    want, _ = _gpu_project(shapes, pg)
+    limit, empty, asked = int(_lib.lib().aprict_b200_project_forbild_scratch_bytes(views, 30)), torch.empty, []
+
+    def short(*a: object, **k: object) -> torch.Tensor:
+        if k.get("dtype") == torch.uint8:
+            asked.append(a[0])
+            if a[0] > limit:
+                raise torch.cuda.OutOfMemoryError
+        return empty(*a, **k)
+
+    monkeypatch.setattr(torch, "empty", short)
+    got, _ = _gpu_project(shapes, pg)
+    assert asked and asked[0] > limit
+    np.testing.assert_array_equal(got, want)
