@@ -1,8 +1,8 @@
 """Launch-shape autotuner.
 
 Times a few candidate launch shapes of the forward projector (detector tile
-height, warp patch shape, neighbouring views per tile) and the backprojector (voxels per thread, size of the brick-ordered
-wave) on the caller's own problem with CUDA events, keeps the fastest, and
+height, warp patch shape, neighbouring views per tile) and the backprojector (voxels per thread and size of the brick-ordered
+wave, of the z columns or the bricks) on the caller's own problem with CUDA events, keeps the fastest, and
 applies it through ``aprict_b200_set_tuning``. Results never depend on these
 knobs; only speed does. Choices are cached per problem signature (in memory,
 and optionally in a JSON file).
@@ -26,6 +26,7 @@ FP_WARP_V = (8, 16, 32)
 FP_VIEWS = ((1, 1), (2, 1), (2, 2), (4, 1), (4, 2))  # (views per tile, views inside a warp)
 BP_XB = (2, 4, 8)
 BP_WAVE = (2, 3, 4, 6)
+KERNELS = 2  # raised when a knob comes to mean another kernel's launch shape: older cache entries are not taken
 
 _cache: dict[str, dict] = {}
 _lock = threading.Lock()
@@ -75,9 +76,11 @@ def _time(fn, reps: int = 3) -> float:
 
 
 def signature(projs: fp.ProjectionSet, volume: Volume, cfg_bp: fp.ConfigBackproject | None) -> str:
-    """Cache key: data shapes, volume order and the backprojection settings."""
+    """Cache key: data shapes and strides, volume order, the backprojection settings and, as they choose the
+    kernel that the knobs apply to, whether the views are upright."""
     c = None if cfg_bp is None else cfg_bp.contents.tobytes().hex()
-    return json.dumps([list(projs.data.shape), list(volume.shape), volume.order, c])
+    kind = None if cfg_bp is None else projs._backproject_promise(cfg_bp.needs_z)  # noqa: SLF001
+    return json.dumps([KERNELS, list(projs.data.shape), list(projs.data.stride()), list(volume.shape), volume.order, c, kind])
 
 
 def tune(

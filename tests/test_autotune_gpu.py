@@ -17,7 +17,7 @@ import torch
 
 from aprict_b200 import Volume, autotune, phantoms
 from aprict_b200.cb import flatpanel as fp
-from helpers import circular, rel_l2
+from helpers import circular, jittered, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -105,3 +105,21 @@ def test_tune_picks_allowed_values_and_caches(restore_knobs, tmp_path) -> None:
     assert cache.exists()
     autotune.apply({})
     assert autotune.tune(ps, vol, cfg_bp=fp.ConfigBackproject(), cache_file=cache) == choice
+
+
+def test_cache_key_tells_the_kernels_apart(restore_knobs, tmp_path) -> None:
+    """Upright and tilted views of one shape take different kernels, as strides may: a choice timed on one is not taken
+    for the other, nor one that an older version left in the file."""
+    import json
+
+    vol, pg = _problem()
+    cfg = fp.ConfigBackproject(fast_approx=True)
+    data = torch.zeros((16, 52, 56), device="cuda")
+    sets = [fp.ProjectionSet(pg, data=data), fp.ProjectionSet(jittered(np.random.default_rng(1), pg), data=data),
+            fp.ProjectionSet(pg, data=data.transpose(1, 2).contiguous().transpose(1, 2))]
+    assert len({autotune.signature(p, vol, cfg) for p in sets}) == 3
+    old = json.dumps([[16, 52, 56], list(SHAPE), "C", cfg.contents.tobytes().hex()])
+    cache = tmp_path / "tune.json"
+    cache.write_text(json.dumps({old: {"bp_xb": 2, "bp_wave": 16}}))
+    assert autotune.tune(sets[0], vol, cfg_bp=cfg, cache_file=cache)["bp_wave"] in autotune.BP_WAVE
+    assert old in json.loads(cache.read_text())
