@@ -108,6 +108,8 @@ SIGNATURES: dict[str, tuple[object, list[object]]] = {
          ctypes.c_uint32, _c_void_p],
     ),
     "aprict_b200_sirt_step": (_c_int, [_c_void_p] * 9 + [_c_void_p]),
+    "aprict_b200_sirt_step_views": (_c_int, [_c_void_p] * 8 + [ctypes.c_uint32, _c_void_p, _c_void_p]),
+    "aprict_b200_sirt_graph_create_views": (_c_int, [_c_void_p] * 8 + [ctypes.c_uint32, _c_void_p, _c_int, _c_void_p]),
     "aprict_b200_sirt_graph_create": (_c_int, [_c_void_p] * 9 + [_c_int, _c_void_p]),
     "aprict_b200_sirt_graph_launch": (_c_int, [_c_void_p, _c_void_p]),
     "aprict_b200_sirt_graph_iterations": (_c_int, [_c_void_p]),

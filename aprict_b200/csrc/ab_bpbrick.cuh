@@ -266,13 +266,14 @@ __device__ __forceinline__ float zpow(const BPParams &P, const ab_bpview &b, flo
 __device__ __forceinline__ bool all_upright(const BPParams &P) {
     if (P.views != (int)APRICT_VIEWS_UNKNOWN) return P.views == (int)APRICT_VIEWS_UPRIGHT;
     const bool needZ = P.pL != 0 || P.pV != 0 || P.preset != 0;
-    bool tilted = false;
-    for (uint32_t v = threadIdx.x; v < P.n_views; v += kThreads) {
+    auto tilted = [&](uint32_t v) {
         const aprict_proj_spec &sp = P.specs[v];
-        tilted = tilted || !(sp.det_u.z == 0.f && sp.det_v.x == 0.f && sp.det_v.y == 0.f) ||
-                 (needZ && sp.det_pos.z != sp.source_pos.z);
-    }
-    return !__syncthreads_or(tilted);
+        return !(sp.det_u.z == 0.f && sp.det_v.x == 0.f && sp.det_v.y == 0.f) || (needZ && sp.det_pos.z != sp.source_pos.z);
+    };
+    if (P.n_views > 0 && tilted(0)) return false;  // most scans that are not upright
+    bool any = false;
+    for (uint32_t v = threadIdx.x; v < P.n_views; v += kThreads) any = any || tilted(v);
+    return !__syncthreads_or(any);
 }
 
 // Block coordinates of work unit `unit`; false past the volume (super-bricks

@@ -465,7 +465,7 @@ APRICT_API int aprict_b200_project_forbild_scratch(const aprict_proj_spec *specs
                                                    aprict_stream_t stream);
 
 /* ---- SIRT (reference mode) ----
- * One iteration of SIRT_flatpanel (sirt_vram.py:130-152) as two launches on
+ * One iteration of SIRT_flatpanel (sirt_vram.py:130-152) on
  * the stream: r = b - A x (fused residual), then x += M (.) B r with cfg_bp
  * (which must apply the summand multiplier M). b, r: projection stacks with
  * the layout of pd; x, M: volumes of vd. */
@@ -473,6 +473,14 @@ APRICT_API int aprict_b200_sirt_step(const aprict_proj_spec *specs_dev, const ap
                                      const float *b_dev, float *r_dev, const aprict_vol_desc *vd, float *x_dev,
                                      const float *M_dev, const aprict_backproject_config *cfg_bp,
                                      uint32_t *status_dev, aprict_stream_t stream);
+
+/* The same with what the caller knows of the views (as in
+ * aprict_b200_backproject_views): two launches instead of three where the
+ * faster kernel for upright views may run. */
+APRICT_API int aprict_b200_sirt_step_views(const aprict_proj_spec *specs_dev, const aprict_proj_desc *pd,
+                                           const float *b_dev, float *r_dev, const aprict_vol_desc *vd, float *x_dev,
+                                           const float *M_dev, const aprict_backproject_config *cfg_bp, uint32_t views,
+                                           uint32_t *status_dev, aprict_stream_t stream);
 
 /* n_iter SIRT steps captured once as a CUDA graph (on a private stream) and
  * replayed with aprict_b200_sirt_graph_launch. The graph records the
@@ -485,6 +493,11 @@ APRICT_API int aprict_b200_sirt_graph_create(const aprict_proj_spec *specs_dev, 
                                              float *x_dev, const float *M_dev,
                                              const aprict_backproject_config *cfg_bp, uint32_t *status_dev,
                                              int n_iter, aprict_sirt_graph **out);
+APRICT_API int aprict_b200_sirt_graph_create_views(const aprict_proj_spec *specs_dev, const aprict_proj_desc *pd,
+                                                   const float *b_dev, float *r_dev, const aprict_vol_desc *vd,
+                                                   float *x_dev, const float *M_dev,
+                                                   const aprict_backproject_config *cfg_bp, uint32_t views,
+                                                   uint32_t *status_dev, int n_iter, aprict_sirt_graph **out);
 APRICT_API int aprict_b200_sirt_graph_launch(const aprict_sirt_graph *graph, aprict_stream_t stream);
 APRICT_API int aprict_b200_sirt_graph_iterations(const aprict_sirt_graph *graph);
 APRICT_API void aprict_b200_sirt_graph_destroy(aprict_sirt_graph *graph);

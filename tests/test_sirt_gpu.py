@@ -212,3 +212,39 @@ def test_c_abi_sirt_step_and_graph_equal_the_python_iterator() -> None:
         lib.aprict_b200_sirt_graph_destroy(g)
     with pytest.raises(ValueError):
         _lib.check(lib.aprict_b200_sirt_step(*args[:6], None, _lib.ptr(cfg), None, stream), "sirt_step")
+
+
+@pytest.mark.parametrize("kind", ["upright", "tilted"])
+def test_c_abi_sirt_with_and_without_a_promise(kind: str) -> None:
+    """A step and a graph of two, with what is known of the views and without: the same kernel's sums."""
+    import ctypes
+
+    from aprict_b200 import _lib
+    from helpers import jittered
+
+    pg, _, b = _problem()
+    if kind == "tilted":
+        pg = jittered(np.random.default_rng(3), pg)
+    lib, stream = _lib.lib(), torch.cuda.current_stream().cuda_stream
+    ps = fp.ProjectionSet(pg, data=b.clone())
+    specs, pd, dptr = fp._view_args(ps, (), 0)  # noqa: SLF001
+    cfg = fp.ConfigBackproject(fast_approx=True, apply_summand_multiplier=True).contents
+    M = Volume.zeros(SHAPE, voxwid=1.0)  # noqa: N806
+    M.fill(1e-5)
+    out = []
+    for views in (0, ps._backproject_promise(False)):  # noqa: SLF001
+        x, r = Volume.zeros(SHAPE, voxwid=1.0), torch.zeros_like(b)
+        vd = x._desc()  # noqa: SLF001
+        args = (specs, _lib.ptr(pd), dptr, r.data_ptr(), _lib.ptr(vd), x.data.data_ptr(), M.data.data_ptr(), _lib.ptr(cfg), views, None)
+        _lib.check(lib.aprict_b200_sirt_step_views(*args, stream), "sirt_step")
+        torch.cuda.synchronize()
+        g = ctypes.c_void_p()
+        _lib.check(lib.aprict_b200_sirt_graph_create_views(*args, 2, ctypes.byref(g)), "sirt_graph_create")
+        _lib.check(lib.aprict_b200_sirt_graph_launch(g, stream), "sirt_graph_launch")
+        torch.cuda.synchronize()
+        lib.aprict_b200_sirt_graph_destroy(g)
+        out.append(x.as_numpy())
+    assert np.linalg.norm(out[0]) > 0
+    np.testing.assert_array_equal(out[0], out[1])
+    with pytest.raises(ValueError):
+        _lib.check(lib.aprict_b200_sirt_step_views(*args[:8], 4, None, stream), "sirt_step")
