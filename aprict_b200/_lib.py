@@ -196,11 +196,17 @@ def upload(a: np.ndarray):  # noqa: ANN201
     return host.to(torch.device("cuda", torch.cuda.current_device()), non_blocking=True)
 
 
-def ptr(a: np.ndarray) -> ctypes.c_void_p:
+def ptr(a: np.ndarray):  # noqa: ANN201
     """Pointer to a numpy array's data (struct arguments are passed by
     pointer). The pointer object holds a reference to the array, so a
-    temporary array stays alive for the duration of the call it is passed to."""
-    return a.ctypes.data_as(ctypes.c_void_p)
+    temporary array stays alive for the duration of the call it is passed to.
+
+    From the array's buffer, at 0.9 us; arrays without a writable one take
+    numpy's ``data_as`` (2.2 us, three of them a good part of a small call)."""
+    try:
+        return ctypes.byref(ctypes.c_char.from_buffer(a))
+    except (TypeError, ValueError, BufferError):  # read-only, empty or not contiguous
+        return a.ctypes.data_as(ctypes.c_void_p)
 
 
 def vol_desc(shape: tuple[int, int, int], order: str, voxwid: float, corner: np.ndarray) -> np.ndarray:

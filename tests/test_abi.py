@@ -246,3 +246,24 @@ def test_batch_plan_refuses_unknown_view_promises(exact: int) -> None:
     rc = lib.aprict_b200_batch_plan_views(1, _lib.ptr(scans), 2, _lib.ptr(confs), _lib.ptr(views), plan.ctypes.data, nbytes)
     assert rc == 1
     assert b"promise" in lib.aprict_b200_last_error()
+
+
+def test_pointers_of_arrays() -> None:
+    """Writable, read-only, empty and strided arrays: the address that numpy gives, and the array kept alive."""
+    import gc
+    import weakref
+
+    take = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p)(lambda p: p)
+    plain, fixed = np.zeros((), S.vol_desc), np.arange(5.0)
+    fixed.setflags(write=False)
+    for a in (plain, np.zeros(3, S.proj_spec), fixed, np.arange(12.0)[1::3], np.arange(12.0)[3:], np.zeros(1, np.uint32)):
+        assert take(_lib.ptr(a)) == a.ctypes.data
+    take(_lib.ptr(np.zeros(0, np.uint8)))
+    a = np.zeros(4)
+    p, ref = _lib.ptr(a), weakref.ref(a)
+    del a
+    gc.collect()
+    assert ref() is not None
+    del p
+    gc.collect()
+    assert ref() is None
