@@ -45,8 +45,9 @@ AB_HD bool ab_finite3(ab_d3 a) { return isfinite(a.x) && isfinite(a.y) && isfini
 // approximate reciprocal or reciprocal square root (relative error 2^-19.9 seen)
 // and one step of Householder's third-order iteration (Householder, "The
 // numerical treatment of a single nonlinear equation", 1970), which leaves
-// e^3 and the last places: within 1 unit of the rounded results on 6.7e7 values
-// between 2^-300 and 2^300. Fewer than half the instructions of the general
+// e^3 and the last places: within 1 unit of the rounded results on 4e6 values
+// between 2^-996 (sqrt: 2^-300) and 2^300, the powers of two and their neighbours
+// (tests/test_forbild.py). Fewer than half the instructions of the general
 // division and square root, whose range checks are not needed here.
 AB_DEV double ab_rcp_h3(double x) {
     double y;

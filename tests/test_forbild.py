@@ -171,6 +171,53 @@ def test_gpu_fan_and_empty() -> None:
 
 
 # ------------------------------------------------- polynomial forms of the ray
+_SEED_PROBE = """
+#include "ab_common.cuh"
+__global__ void k(const double *x, double *r, double *s, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        r[i] = ab_rcp_h3(x[i]);
+        s[i] = x[i] > 0.0 ? ab_sqrt_h3(x[i]) : 0.0;
+    }
+}
+extern "C" __attribute__((visibility("default"))) int run(const double *x, double *r, double *s, int n) {
+    k<<<(n + 255) / 256, 256>>>(x, r, s, n);
+    return (int)cudaDeviceSynchronize();
+}
+"""
+
+
+@pytest.mark.gpu
+def test_third_order_steps_on_the_device(tmp_path) -> None:  # noqa: ANN001
+    """ab_rcp_h3 and ab_sqrt_h3 as the kernels compile them: within one unit in the last place of the rounded 1 / x and
+    sqrt(x), over the exponents that the projectors meet (1e-300, the least step along an axis, to 2^300; roots from
+    2^-300), powers of two and their neighbours among them."""
+    import ctypes
+    import subprocess
+
+    import torch
+
+    from aprict_b200 import build
+
+    (tmp_path / "probe.cu").write_text(_SEED_PROBE)
+    lib = tmp_path / "probe.so"
+    subprocess.run([build._nvcc(), *build.ARCH_FLAGS, *build.NVCC_FLAGS, f"-I{build.INCLUDE}", f"-I{build.CSRC}", "-shared",
+                    str(tmp_path / "probe.cu"), "-o", str(lib)], check=True, capture_output=True)
+    run = ctypes.CDLL(str(lib)).run
+    rng = np.random.default_rng(6)
+    two = np.ldexp(1.0, np.arange(-996, 301))
+    x = np.concatenate([np.ldexp(rng.uniform(1, 2, 4_000_000), rng.integers(-996, 300, 4_000_000)), two, np.nextafter(two, 0),
+                        np.nextafter(two, np.inf), [1e-300, -1e-300, 3.0, -7.0]])
+    d, r, s = torch.from_numpy(x).cuda(), *torch.zeros((2, len(x)), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert run(ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(r.data_ptr()), ctypes.c_void_p(s.data_ptr()), len(x)) == 0
+    want = 1.0 / x
+    assert (np.abs(r.cpu().numpy() - want) / np.spacing(np.abs(want))).max() <= 1.0
+    k = x > 2.0**-300
+    want = np.sqrt(x[k])
+    assert (np.abs(s.cpu().numpy()[k] - want) / np.spacing(want)).max() <= 1.0
+
+
 def test_third_order_steps_bound() -> None:
     """One third-order Householder step from a seed good to 2^-19.9 gives 1 / x and sqrt(x) to the seed's error cubed
     (2^-59.7; for the root, with e twice the seed's, 5/16 of 2^-56.7) and the last steps' rounding: 1.5 and 2 units of 2^-53. Same operations, each
