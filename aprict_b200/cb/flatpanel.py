@@ -436,9 +436,10 @@ class ProjectionSet:
     def specs_device(self) -> torch.Tensor:
         """The packed views on the device (uint8 bytes, flattened), cached."""
         if self._specs_dev is None:
-            self._specs_host = self._proj_specs.reshape(-1).copy()
+            raw = np.ascontiguousarray(self._proj_specs.reshape(-1)).view(np.uint8).copy()  # (of bytes: 720 views 3 us, of records 59)
+            self._specs_host = raw.view(S.proj_spec)
             _device()
-            self._specs_dev = _lib.upload(self._specs_host.view(np.uint8))
+            self._specs_dev = _lib.upload(raw)
         return self._specs_dev
 
     def _backproject_promise(self, needs_z: bool) -> int:

@@ -65,14 +65,16 @@ def _compiled(volume: object) -> _Compiled:
     return volume._compiled[1]
 
 
-def _scratch(nbytes: int, least: int, device: torch.device) -> torch.Tensor | None:
-    """Device scratch of ``nbytes``, or what is to be had of it from ``least`` up (the projector
-    takes the views in groups then), or none (its tiles derive the records themselves)."""
-    while nbytes >= max(1, least):
+def _scratch(views: int, shapes: int, device: torch.device) -> torch.Tensor | None:
+    """Device scratch for the per-(view, shape) records, or what is to be had of it from one view's
+    up (the projector takes the views in groups then), or none (its tiles derive the records)."""
+    size = _lib.lib().aprict_b200_project_forbild_scratch_bytes
+    nbytes = int(size(views, shapes))
+    while nbytes > 0:
         try:
             return torch.empty(nbytes, dtype=torch.uint8, device=device)
         except torch.cuda.OutOfMemoryError:
-            nbytes //= 4
+            nbytes = nbytes // 4 if nbytes // 4 >= int(size(1, shapes)) else 0
     return None
 
 
@@ -90,8 +92,7 @@ def project_shapes(config: object, volume: object, projs: object) -> None:
         mode = 0
     counter = projs.out_of_mem_counter
     lib = _lib.lib()
-    size = lib.aprict_b200_project_forbild_scratch_bytes
-    scratch = _scratch(int(size(int(projs.proj_specs.shape[-1]), comp.n)), int(size(1, comp.n)), comp.dev.device)
+    scratch = _scratch(int(projs.proj_specs.shape[-1]), comp.n, comp.dev.device)
     sptr, nbytes = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel())
     for it, first in _leading_slices(projs):
         specs, pd, dptr = _view_args(projs, it, first)
