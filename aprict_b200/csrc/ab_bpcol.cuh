@@ -27,19 +27,19 @@
 // of odd height has its mid plane on the edge between two rows: it is set to 0,
 // queued per warp and settled with up to 31 others, one per lane, its product going
 // to the voxel's compensated total. 255^3 x 120 views, mid plane and axis on edges:
-// 2.15 ms (settled at once, by a call in the view loop: 3.83 ms; 256^3 x 180 views,
+// 2.14 ms (settled at once, by a call in the view loop: 3.83 ms; 256^3 x 180 views,
 // no edges: 1.69 and 1.82 ms).
 //
 // Bound: gather latency and issue (on 256^3 x 360 views x 384^2 nearest: 12.5
 // warp instructions per 32 voxel-views against 21 of the brick kernel's z-lane
 // path before it, issue 54 %, L1 wavefronts 60 %). Measured there, four CTAs per
-// SM: nearest 4.93 -> 3.11 ms (F order 14.8 -> 3.3 ms: its lanes gathered 32
-// pixel columns), direct raycast 13.8 -> 3.1 ms; 64^3 x 90 views 72 -> 55 us;
-// bilinear on 210 x 190 x 150 x 200 views 2.06 -> 1.73 ms. Three CTAs at 80
-// registers, no spills: 3.6 ms.
+// SM, no mask: nearest 6.73 -> 4.36 ms (F order 16.6 -> 4.5 ms: its lanes gathered
+// 32 pixel columns), direct raycast 17.1 -> 4.4 ms; 64^3 x 90 views 115 -> 44 us;
+// bilinear on 210 x 190 x 150 x 200 views 2.90 -> 2.20 ms. Three CTAs at 80
+// registers, no spills: a sixth slower. Which calls take it: columns_pay.
 //
 // Columns cut by the detector's edges (helical scans; 256^3 x 180 views, one
-// turn): nearest 6.4 -> 2.5 ms, direct raycast 7.7 -> 2.6 ms. Their blocks are
+// turn): nearest 7.4 -> 2.9 ms, direct raycast 7.7 -> 2.9 ms. Their blocks are
 // gathered under a predicate (a branch around the gather: twice the time), blocks
 // inside four at a time.
 #pragma once

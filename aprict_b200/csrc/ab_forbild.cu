@@ -569,8 +569,8 @@ __device__ __noinline__ bool ray_interval_general(const QView &q, double fu, dou
 // that misses the solid by more than rounding ends after the discriminant, and the cylinder's caps
 // and the clip planes divide only where they cut the interval found so far.
 // A miss costs 7 FP64 operations (the direction, A, B and C first: some 25), a
-// hit's two roots no division: 240 views x 1024^2 of 100 clipped quadrics 15.4 ->
-// 13.4 ms.
+// hit's two roots no division: 240 views x 1024^2 of 100 clipped quadrics 15.4-19.2 ->
+// 13.5-14.1 ms.
 __device__ __forceinline__ bool ray_interval(const QView &q, double fu, double fv, double &lo, double &hi) {
     if (!q.fast) return ray_interval_general(q, fu, fv, lo, hi);
     const double a = fu - q.uc, b = fv - q.vc;

@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
 // 6000 heights: 0.045 at most). Where that exceeds kTol, a third of the samples'
 // FP32 rounding, and below 128 h, the heights are summed directly, as in calls
 // without scratch for the table.
-// 396 radii x 6000 x 6000 samples, the whole call: 7.0 -> 0.55 ms (most of it host
+// 396 radii x 6000 x 6000 samples, the whole call: 7.0 -> 0.53-0.68 ms (most of it host
 // work; sums equal to 1e-8).
 // sin^2 theta grows with z, so a height sum stops at the first height past the
 // vertical window, where the window is 0 (it reaches 0 continuously at its

@@ -2,8 +2,9 @@
 source locus (drop-in for src/aprict/gbc/weightinteg.py:22-91).
 
 The integral over source heights and angles is evaluated by
-``aprict_b200_gbc_weight_integral`` (one thread per (height, angle) sample,
-FP64 block sums); the xy-grid form interpolates it linearly in the radius.
+``aprict_b200_gbc_weight_integral_scratch`` (the sums over heights at the
+nodes of a table, one thread per (radius, angle), FP64 block sums); the
+xy-grid form interpolates it linearly in the radius.
 """
 
 from __future__ import annotations
