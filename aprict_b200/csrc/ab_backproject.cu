@@ -76,7 +76,7 @@ extern "C" int aprict_b200_backproject_views(const aprict_proj_spec *specs_dev, 
     P.views = (int)views;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const bool lin = cfg->approx_mode_linear_interpolate != 0;
-    if (cxb != 0 && views != APRICT_VIEWS_MIXED && !columns_pay(vd, cfg, col_units_of(vd, cxb), false)) P.views = (int)(views = APRICT_VIEWS_GENERAL);
+    if (cxb != 0 && views != APRICT_VIEWS_MIXED && !columns_pay(vd, pd->n_views, cfg, col_units_of(vd, cxb), false)) P.views = (int)(views = APRICT_VIEWS_GENERAL);
     if (cxb != 0 && (views == APRICT_VIEWS_UNKNOWN || views == APRICT_VIEWS_UPRIGHT)) {
         const bool ray = cfg->approx_mode_direct_raycast != 0;
         if (cxb == 8)

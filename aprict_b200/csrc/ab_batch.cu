@@ -373,8 +373,8 @@ extern "C" int aprict_b200_batch_plan_views(int op, const aprict_scan *scans, in
     for (int i = 0; i < n_scans; ++i)
         if (col(i)) col_units += ab_bp::col_units_of(&scans[i].vol, plan_cxb);
     for (int i = 0; i < n_scans; ++i) {
-        if (col(i) && !ab_bp::columns_pay(&scans[i].vol, static_cast<const aprict_backproject_config *>(configs) + i,
-                                          col_units, true))
+        if (col(i) && !ab_bp::columns_pay(&scans[i].vol, scans[i].projs.n_views,
+                                          static_cast<const aprict_backproject_config *>(configs) + i, col_units, true))
             kind[i] = APRICT_VIEWS_GENERAL;
         cols = cols || col(i);
         bricks = bricks || kind[i] != APRICT_VIEWS_UPRIGHT;

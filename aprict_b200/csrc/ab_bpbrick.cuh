@@ -1257,17 +1257,28 @@ inline int bp_sms() {
 //   C order  nz 8: 1055, 586   32: 1059, 599   40: 1180, 1122   64: 678, 1070
 //            (detectors that do not, nz 40: 656, 1005)
 //   F order  nz 8: 1061, 229   40: 1212, 748   48: 1212, 870   56: 947, 1026
+//            nz 64: 763, 1122   96: 1510, 1607 (a second pair of blocks: 65 costs what 96
+//            does, in bricks some 1130)
 // 64^2 (one wave: 512 CTAs) x 24: 89, 126 (C), 90, 100 (F); 64^2 x 2: 88, 90 (C), 89, 83 (F).
+// In F order a column's lanes read and write the volume 4 bytes a line, which few views
+// do not pay for: 128^3 from 4 views 121, 55, from 16 136, 122; 256^3 from 10 672, 569;
+// bilinear, 64^3 from 8 31, 33, from 10 31, 39; 128^3 from 4 125, 89.
 // Batches fill the GPU with bricks too (and skip views off a brick). 6 x 128^2 x nz:
-//   C order, nearest    nz 48: 1837, 1551   56: 1347, 1452   96: 2205, 1966
+//   C order, nearest    nz 48: 1837, 1551   56: 1347, 1452   96: 2205, 1966   100: 2571, 2808
 //   C order, bilinear   nz 32: 1737, 831    48: 2531, 2988   96: 2291, 2398
 //   F order, nearest    nz 96: 2286, 2046   112: 1886, 2385
 //   F order, bilinear   nz 48: 2554, 1861   56: 1860, 2395
-inline bool columns_pay(const aprict_vol_desc *vd, const aprict_backproject_config *cfg, uint64_t col_units, bool batch) {
+constexpr uint32_t kSecondPair = 88;  // layers from which a second pair of blocks pays where the bricks' cost is the height's
+inline uint32_t views_f(const aprict_backproject_config *cfg) { return cfg->approx_mode_linear_interpolate ? 8 : 16; }  // F order pays above
+inline bool columns_pay(const aprict_vol_desc *vd, uint32_t n_views, const aprict_backproject_config *cfg, uint64_t col_units,
+                        bool batch) {
     const uint64_t wave = (uint64_t)kColBlocks * (uint64_t)bp_sms();
-    if (vd->order == 0) return vd->nz > (batch ? 48u : 32u) || col_units <= wave;
     const bool nearest = !cfg->approx_mode_direct_raycast && !cfg->approx_mode_linear_interpolate;
-    return vd->nz > (batch && nearest ? 104u : 48u) || col_units <= wave * 3 / 4;
+    const uint32_t nz = vd->nz;
+    if (vd->order == 0)
+        return col_units <= wave || (batch ? nz > 48u && !(nearest && nz > 64u && nz <= 96u) : nz > 32u);
+    return n_views > views_f(cfg) && (col_units <= wave * 3 / 4 || (batch && nearest ? nz > 104u : nz > 48u &&
+                                 !(nearest && nz > 64u && nz < kSecondPair)));
 }
 
 // Voxels per thread of the z-column kernel: the fewest that hold the column

@@ -1093,11 +1093,13 @@ extern "C" int aprict_b200_backproject_gbc_views(const aprict_proj_spec *specs_d
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const int order_f = vd->order != 0;
     // C order: the columns at every size. F order: its lanes along x have a flat volume's
-    // voxels side by side and need no column, and a small one's are too few for 8 voxels a
-    // lane. 198^2 x nz from 120 views bilinear, columns and k_backproject_gbc: 8: 1096, 292 us;
-    // 48: 1557, 1470; 64: 791, 1971; 24^2 x 100: 164, 79; 48^2 x 64: 91, 157.
+    // voxels side by side and need no column, a small one's are too few for 8 voxels a
+    // lane, and a column reads and writes both volumes 4 bytes a line. 198^2 x nz from 120
+    // views bilinear, columns and k_backproject_gbc: 8: 1096, 292 us; 48: 1557, 1470; 64:
+    // 791, 1971; 24^2 x 100: 164, 79; 48^2 x 64: 91, 157; nearest 99^2 x 65: 455, 383.
     if (cxb != 0 && order_f &&
-        !(vd->nz > 48u && ab_bp::col_units_of(vd, kGCol) >= 3 * (uint64_t)ab_bp::bp_sms() / 2))
+        !(pd->n_views > ab_bp::views_f(cfg) && vd->nz > 48u && !(vd->nz > 64u && vd->nz < ab_bp::kSecondPair) &&
+          ab_bp::col_units_of(vd, kGCol) >= 3 * (uint64_t)ab_bp::bp_sms() / 2))
         P.views = (int)(views = APRICT_VIEWS_GENERAL);
     if (cxb != 0 && views != APRICT_VIEWS_GENERAL) {
         // The window's flat part and its end as bounds on |z - s_z| / (R ell),

@@ -211,8 +211,8 @@ def knob():
 def test_flat_volumes_on_both_sides_of_the_rule(mode: str, order: str, knob) -> None:  # noqa: ANN001
     """Volumes of more columns than one wave of CTAs: flat ones take the bricks, tall ones the columns; at every
     height the call gives what either kernel gives, alone and in a batch with others of other kinds."""
-    shapes = [(90, 71, nz) for nz in (2, 31, 32, 33, 48, 49)]
-    pgs = [circular(10, 300, 200, 1.37, 77, max(12, int(0.9 * s[2]))) for s in shapes]
+    shapes = [(90, 71, nz) for nz in (2, 31, 32, 33, 48, 49, 64, 65, 88, 97, 105)]
+    pgs = [circular(m, 300, 200, 1.37, 77, max(12, int(0.9 * s[2]))) for s, m in zip(shapes, (17, 16, 17, 16, 17, 17, 8, 17, 9, 17, 17))]
     datas = [_data(g, i) for i, g in enumerate(pgs)]
     tol = 1e-5 if mode == "bilinear" else 1e-6
     auto, bricks = [], []

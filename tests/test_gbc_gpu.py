@@ -277,9 +277,9 @@ def test_gbc_reconstruction_matches_oracle() -> None:
 
 @pytest.mark.parametrize("linear", [False, True])
 @pytest.mark.parametrize("order", ["C", "F"])
-@pytest.mark.parametrize("shape", [(12, 11, 9), (40, 40, 48), (40, 40, 49), (50, 48, 49), (50, 48, 40)])
+@pytest.mark.parametrize("shape", [(12, 11, 9), (40, 40, 48), (40, 40, 49), (50, 48, 49), (50, 48, 64), (50, 48, 65), (50, 48, 88)])
 def test_every_kernel_gives_the_same(shape: tuple, order: str, linear: bool) -> None:
-    """F-order volumes take the columns above 48 layers and 222 CTAs, C-order ones at every size: without a promise,
+    """F-order volumes take the columns from 49 to 64 and from 88 layers, above 222 CTAs, C-order ones at every size: without a promise,
     with it, and with the general kernel, all to FP32 rounding (bilinear: the general kernels' coordinates are FP32); a scan with one tilted view takes the general kernel also without a promise."""
     pg = _scan(m=20, h=8.0, nu=61, nv=50)
     vecs = {k: np.broadcast_to(getattr(pg, k), (20, 3)).copy() for k in ("source_pos", "det_pos", "det_uvec", "det_vvec")}
