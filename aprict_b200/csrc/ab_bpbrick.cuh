@@ -102,6 +102,12 @@ __device__ __forceinline__ int round_index(float x, float lo, float hi, float &f
     return __float_as_int(t) - 0x4B400000;
 }
 
+// Offset of sub-sample i along an axis, in voxels from the voxel's centre; off: 1 over their number. The
+// bricks, the columns and the GBC kernels take this one, rounded so: where a voxel
+// projects exactly on the edge between two pixels (the middle one of three sub-samples
+// in the mid plane of an odd grid), 1.5e-8 of a voxel decides.
+__device__ __forceinline__ float sub_offset(float off, int i) { return fmaf(off, 0.5f + (float)i, -0.5f); }
+
 // FP64 position of a voxel (centre + sub-sample offset) relative to the
 // volume centre, from its integer indices: exact in double.
 struct VoxRef {
@@ -515,6 +521,7 @@ __device__ __forceinline__ void bp_brick(const BPParams &P, uint32_t brick,
         const int si = isub / (P.ssy * P.ssz), sj = (isub / P.ssz) % P.ssy, sk = isub % P.ssz;
         {
             {
+                // (sub_offset's rounding: the compiler contracts them)
                 const float fsub[3] = {-0.5f + offx * (0.5f + si), -0.5f + offy * (0.5f + sj),
                                        -0.5f + offz * (0.5f + sk)};
                 const float X0 = base[0] + fsub[0] * vw, Y0 = base[1] + fsub[1] * vw, Z0 = base[2] + fsub[2] * vw;

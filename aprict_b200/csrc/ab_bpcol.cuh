@@ -236,9 +236,9 @@ __device__ __forceinline__ void bp_columns(const BPParams &P, uint32_t brick, Co
         sm.par.sv4 = sv4;
     }
     for (int isub = 0; isub < n_sub; ++isub) {
-        const double fx = -0.5 + (0.5 + isub / (P.ssy * P.ssz)) / P.ssx;
-        const double fy = -0.5 + (0.5 + (isub / P.ssz) % P.ssy) / P.ssy;
-        const double fz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
+        const double fx = sub_offset(1.f / (float)P.ssx, isub / (P.ssy * P.ssz));
+        const double fy = sub_offset(1.f / (float)P.ssy, (isub / P.ssz) % P.ssy);
+        const double fz = sub_offset(1.f / (float)P.ssz, isub % P.ssz);
         // the column's first voxel relative to the volume centre
         // (kept in shared memory: the view loop has no registers for it)
         if (lane == 0) {

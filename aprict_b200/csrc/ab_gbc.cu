@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kGThreads, BILIN ? 3 : 4) k_backproject_gbc(co
             float fsub[3], rel[3], wp[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                fsub[a] = -0.5f + offs[a] * (0.5f + (float)sidx[a]);
+                fsub[a] = -0.5f + offs[a] * (0.5f + (float)sidx[a]);  // sub_offset, contracted
                 // relative to the volume centre, for the detector coordinate
                 rel[a] = ((float)id[a] + 0.5f - 0.5f * (float)P.n[a]) * vw + fsub[a] * vw;
                 // world position as the reference forms it (pos_000_c + idx voxwid + offset voxwid)
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kGThreads, BILIN ? 3 : 4) k_backproject_gbc_z(
             const int sidx[3] = {isub / (P.ssy * P.ssz), (isub / P.ssz) % P.ssy, isub % P.ssz};
             float fsub[3];
 #pragma unroll
-            for (int a = 0; a < 3; ++a) fsub[a] = -0.5f + offs[a] * (0.5f + (float)sidx[a]);
+            for (int a = 0; a < 3; ++a) fsub[a] = -0.5f + offs[a] * (0.5f + (float)sidx[a]);  // sub_offset, contracted
             const int idv[2] = {ix, iy};
             float rel[2], wp[2];
 #pragma unroll
@@ -458,6 +458,7 @@ struct GbcColSmem {
     GbcView view[kGChunk];
     GbcRec rec[kGThreads / 32][32];
     float vol[kGThreads / 32][32 * kGCol], wsum[kGThreads / 32][32 * kGCol];
+    double pos[kGThreads / 32][4];  // the warp's column, as ColSmem's
 };
 
 template <bool BILIN>
@@ -488,15 +489,18 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
     const int n_sub = P.ssx * P.ssy * P.ssz;
 
     for (int isub = 0; isub < n_sub; ++isub) {
-        const double ox = -0.5 + (0.5 + isub / (P.ssy * P.ssz)) / P.ssx;
-        const double oy = -0.5 + (0.5 + (isub / P.ssz) % P.ssy) / P.ssy;
-        const double oz = -0.5 + (0.5 + isub % P.ssz) / P.ssz;
-        const double X = (ix + 0.5 + ox - 0.5 * P.n[0]) * P.vwd, Y = (iy + 0.5 + oy - 0.5 * P.n[1]) * P.vwd;
-        const double zi0 = z0 + 0.5 + oz - 0.5 * P.n[2], Z0 = zi0 * P.vwd;
+        const float ox = sub_offset(1.f / (float)P.ssx, isub / (P.ssy * P.ssz));
+        const float oy = sub_offset(1.f / (float)P.ssy, (isub / P.ssz) % P.ssy);
+        const float oz = sub_offset(1.f / (float)P.ssz, isub % P.ssz);
+        if (lane == 0) {
+            sm.pos[warp][0] = (ix + 0.5 + ox - 0.5 * P.n[0]) * P.vwd;
+            sm.pos[warp][1] = (iy + 0.5 + oy - 0.5 * P.n[1]) * P.vwd;
+            sm.pos[warp][2] = z0 + 0.5 + oz - 0.5 * P.n[2];
+        }
         // world position of the column's first voxel
-        const float wx = (G.pos000[0] + (float)ix * P.voxwid) + (float)ox * P.voxwid;
-        const float wy = (G.pos000[1] + (float)iy * P.voxwid) + (float)oy * P.voxwid;
-        const float wz = (G.pos000[2] + (float)z0 * P.voxwid) + (float)oz * P.voxwid;
+        const float wx = (G.pos000[0] + (float)ix * P.voxwid) + ox * P.voxwid;
+        const float wy = (G.pos000[1] + (float)iy * P.voxwid) + oy * P.voxwid;
+        const float wz = (G.pos000[2] + (float)z0 * P.voxwid) + oz * P.voxwid;
         for (uint32_t v0 = 0; v0 < P.n_views; v0 += kGChunk) {
             const int cn = (int)min((uint32_t)kGChunk, P.n_views - v0);
             __syncthreads();
@@ -551,6 +555,7 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
                             unsigned in = 0, across = 0, cols = 0;
                             float Af = 0.f, Sf = 0.f, du = 0.f, eps = 0.f;
                             uint64_t col = 0;
+                            const double X = sm.pos[warp][0], Y = sm.pos[warp][1], Z0 = sm.pos[warp][2] * P.vwd;
                             const double D = fma(gv.d.den[0], X, fma(gv.d.den[1], Y, gv.d.den[3]));
                             const double rD = 1.0 / D;
                             const double fu = fma(gv.d.nu[0], X, fma(gv.d.nu[1], Y, gv.d.nu[3])) * rD;
@@ -636,6 +641,7 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
                             if (fmaxf(fabsf(da), fabsf(db)) > ra.z) {
                                 upk(f, fa, fb);
                                 const ab_bpview_d &vd = sm.view[g0 + j].d;
+                                const double X = sm.pos[warp][0], Y = sm.pos[warp][1], zi0 = sm.pos[warp][2];
                                 if (fabsf(da) > ra.z)
                                     pa = col_exact_row(vd, X, Y, (zi0 + (double)(lane + 64 * k)) * P.vwd, fa, crow, (int)P.nv, col, sv4);
                                 if (fabsf(db) > ra.z)
@@ -688,8 +694,8 @@ __global__ void __launch_bounds__(kGThreads, 4) k_backproject_gbc_columns(const 
                         } else {
                             const float t = __fadd_rn(f, kMagic);
                             if (fabsf(__fsub_rn(f, __fsub_rn(t, kMagic))) > ra.z)
-                                pv = col_exact_row(sm.view[g0 + j].d, X, Y, (zi0 + (double)(lane + 32 * k)) * P.vwd, f, crow,
-                                                   (int)P.nv, col, sv4);
+                                pv = col_exact_row(sm.view[g0 + j].d, sm.pos[warp][0], sm.pos[warp][1],
+                                                   (sm.pos[warp][2] + (double)(lane + 32 * k)) * P.vwd, f, crow, (int)P.nv, col, sv4);
                             else if ((unsigned)(__float_as_int(t) - 0x4B400000 + crow) < P.nv)
                                 pv = __ldg(reinterpret_cast<const float *>(col + (uint64_t)(uint32_t)__float_as_int(t) * sv4));
                         }

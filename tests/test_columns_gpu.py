@@ -279,3 +279,20 @@ def test_promise_is_of_the_uploaded_views() -> None:
     v = Volume.zeros(shape, voxwid=1.0)
     fp.backproject(fp.ConfigBackproject(**MODES["nearest"]), v, ps, block=True)
     np.testing.assert_array_equal(v.as_numpy(), want)
+
+
+@pytest.mark.parametrize("ss", [(1, 1, 3), (3, 1, 1), (2, 2, 3), (1, 3, 2)])
+@pytest.mark.parametrize("mode", ["nearest", "raycast"])
+def test_sub_samples_on_edges_fall_as_in_the_bricks(mode: str, ss: tuple, knob) -> None:  # noqa: ANN001
+    """The middle one of three sub-samples of an odd grid's mid plane or axis lies on the edge between two pixels in
+    every view; its offset, rounded as the general kernel's, decides."""
+    for shape, nu, nv in (((20, 22, 33), 31, 40), ((21, 19, 33), 30, 41), ((21, 23, 7), 30, 40)):
+        pg = circular(40, 160, 120, 0.913, nu, nv, theta0=0.3)
+        data, out = _data(pg, 2), []
+        for value in (0, 1):
+            knob(value)
+            v = Volume.zeros(shape, voxwid=0.5)
+            fp.backproject(fp.ConfigBackproject(**MODES[mode], ssx=ss[0], ssy=ss[1], ssz=ss[2]), v, fp.ProjectionSet(pg, data=data), block=True)
+            out.append(v.as_numpy())
+        assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[1]).max()
+        assert rel_l2(out[0], out[1]) <= 1e-6

@@ -198,7 +198,8 @@ def test_non_finite_pixels_outside_the_window(linear: bool) -> None:
 
 
 @pytest.mark.parametrize(("shape", "nu", "nv"), [((20, 22, 33), 31, 40), ((21, 19, 64), 30, 41)])
-def test_exact_ties_fall_as_in_the_general_kernel(shape: tuple, nu: int, nv: int) -> None:
+@pytest.mark.parametrize("ss", [1, 3])
+def test_exact_ties_fall_as_in_the_general_kernel(shape: tuple, nu: int, nv: int, ss: int) -> None:
     """As the columns' test of the same name: mid plane or axis between two pixels in every view of a circular scan."""
     pg = _scan(m=70, h=0.0, nu=nu, nv=nv)
     projs = np.random.default_rng(3).random((70, nu, nv)).astype(np.float32)
@@ -207,7 +208,7 @@ def test_exact_ties_fall_as_in_the_general_kernel(shape: tuple, nu: int, nv: int
         v, ws = Volume.zeros(shape, voxwid=0.9), Volume.zeros(shape, voxwid=0.9)
         ps = fp.ProjectionSet(pg, data=projs)
         ps._backproject_promise = lambda needs_z, views=views: views  # noqa: SLF001
-        fp.backproject(_cfg(False), v, ps, secondary_volume=ws, block=True)
+        fp.backproject(_cfg(False, ss), v, ps, secondary_volume=ws, block=True)
         out.append(v.as_numpy())
     assert np.linalg.norm(out[1]) > 0
     assert np.abs(out[0] - out[1]).max() <= 1e-5 * np.abs(out[1]).max()
